@@ -9,7 +9,7 @@
 // Both run as kind::f8f6f4 on e4m3 operands with fp32 accumulation in TMEM.
 //   * P is split into two e4m3 terms (~8 significant bits): for 16 / 32 rows P = hi + lo/16 as the two halves of the
 //     MMA's 2N columns, for 64 rows hi and lo (unscaled) are two k-steps into the same columns (side by side, O alone
-//     would fill the 512 TMEM columns).
+//     would fill the 512 TMEM columns); how far below the maximum the eight bits reach: Cfg::P_SCALE_LOG2.
 //   * A bf16 Q is split the same way: Q = (hi + lo/16) / s, s a power of two per group of N rows; the QK MMA then has
 //     2N columns and the softmax adds the two halves.  (No tensor-core kind mixes bf16 with fp8 / fp4 operands.)
 //   * MXFP4 / hybrid cache rows become e4m3 operand bytes in "feed" warps: all blocks of a 16-token unit share one
@@ -29,7 +29,7 @@
 //        (the PV warp, or the first fetch warp, searches the CTA's span before that)
 // What bounds it, and microseconds a call before (a kernel per family, maximum of Q and merge as launches of their own, one
 // issuing warp) and now: e4m3 256 x 8192 the HBM rate (264 -> 216), 128 heads over an e4m3 cache the chain load -> QK -> softmax -> PV
-// of two stages (236 -> 76), MXFP4 64 x 8192 the same chain with the conversion in it (96 -> 67), MXFP4 8 x 131072 with two
+// of two stages (236 -> 86), MXFP4 64 x 8192 the same chain with the conversion in it (96 -> 67), MXFP4 8 x 131072 with two
 // queries conversion and shared memory (214 -> 150), hybrid 128 heads the MMA streams (640 -> 395), e4m3 4 x 1024 latencies (23.5 -> 12.3).
 // Synchronisation is mbarrier based; every wait is bounded and on expiry sets a status word.
 //
@@ -49,8 +49,6 @@ constexpr int NS_MAX = 3;                 // operand stages
 constexpr int UNIT_TOK = 16;              // tokens per unit of the feed warps
 constexpr int RAW_MAX = 10;               // landing buffers of a block-scaled cache
 constexpr int SMEM_LIMIT = 232448;        // opt-in shared memory per CTA
-constexpr float RECENTER = 4.0f;          // log2 units
-constexpr float P_SCALE_LOG2 = 4.0f;      // probabilities are stored multiplied by 2^4
 constexpr int E_BIAS = 127 + 6;           // operand bytes of a block-scaled unit are in units of 2^(E_unit - E_BIAS)
 
 struct Misc {
@@ -87,6 +85,13 @@ struct Cfg {
     static constexpr int STAGE_BYTES = 4 * PANEL_BYTES + ROPE_PANEL_BYTES;
     static constexpr bool MERGED = N == 64;
     static constexpr int OB = MERGED ? N : 2 * N;                 // TMEM columns of one O block
+    // A probability p (relative to the reference maximum) is stored as 2^P_SCALE_LOG2 p; a score more than RECENTER log2 units above
+    // the reference maximum moves it.  2^(P_SCALE_LOG2 + RECENTER) must stay below 448.  The smallest step of the stored pair is
+    // 2^-13 with lo / 16 in columns of its own, 2^-9 where lo shares hi's columns (MERGED): there the larger factor keeps the same
+    // 2^-17 below the reference maximum, at the price of moving it more often (48 ragged sequences of 128 heads: 85.6 us; with
+    // 2^4 74.7, but like keys 12 binades down came out 28 % wrong).  Block-scaled caches at 64 rows keep 2^4, i.e. 2^-13.
+    static constexpr bool DEEP = MERGED && !XF;
+    static constexpr float P_SCALE_LOG2 = DEEP ? 8.0f : 4.0f, RECENTER = DEEP ? 0.75f : 4.0f;
     static constexpr int P_CHUNK_BYTES = TILE * 16;               // 16 columns x TILE tokens
     static constexpr int P_BUF_BYTES = (2 * N / 16) * P_CHUNK_BYTES;
     static constexpr int P_BUFS = XF && N > 16 ? 1 : 2;           // single where the landing buffers need the room
@@ -678,7 +683,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                         for (int c = 1; c < NC - 1; c += 2) xm = max3(xm, x[c], x[c + 1]);
                         xm = fmaxf(xm, x[NC - 1]);
                     }
-                    recenter = named_bar_or(bar_id, 128, xm > P_SCALE_LOG2 + RECENTER);
+                    recenter = named_bar_or(bar_id, 128, xm > C::P_SCALE_LOG2 + C::RECENTER);
                 }
                 // a larger exponent frame than the one O is held in: O moves to the new frame
                 float o_frame = 1.0f;
@@ -698,10 +703,10 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                         named_bar_sync(bar_id, 128);
                         if (tok < NC) {                           // one thread per query row
                             const float mx = fmaxf(fmaxf(ms.red[sg][0][tok], ms.red[sg][1][tok]), fmaxf(ms.red[sg][2][tok], ms.red[sg][3][tok]));
-                            const float m_old = first ? -INFINITY : P_SCALE_LOG2 - ms.nm[sg][nm_cur][tok];     // -inf while the row has seen no key
+                            const float m_old = first ? -INFINITY : C::P_SCALE_LOG2 - ms.nm[sg][nm_cur][tok];     // -inf while the row has seen no key
                             const float m_new = fmaxf(m_old, mx);
                             ms.fac[sg][tok] = (m_new == m_old) ? 1.0f : (m_old == -INFINITY ? 0.0f : ex2(m_old - m_new));
-                            ms.nm[sg][nm_cur ^ 1][tok] = P_SCALE_LOG2 - m_new;
+                            ms.nm[sg][nm_cur ^ 1][tok] = C::P_SCALE_LOG2 - m_new;
                         }
                         nm_cur ^= 1;
                         named_bar_sync(bar_id, 128);
@@ -740,7 +745,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                 if (lane == 0) mbar_arrive(&ms.s_empty[sb]);      // the scores have been read for the last time
                 uint32_t hi[NC / 4], lo[NC / 4];
                 if (active) {
-                    // stored probability = p * 2^4 * 2^(e_unit - e_run): this token's V bytes are in the frame e_unit, O in e_run
+                    // stored probability = p * 2^P_SCALE_LOG2 * 2^(e_unit - e_run): this token's V bytes are in the frame e_unit, O in e_run
                     const float p_frame = C::XF ? pow2i(e_unit - e_run) : 1.0f;
                     const f32x2 pf = pk2(p_frame, p_frame), neg = pk2(-1.0f, -1.0f);
                     // MERGED: the lo term shares O's columns with the hi term, so it carries no factor of its own

@@ -209,3 +209,26 @@ def test_two_streams_and_threads_with_one_shape(pkg):
     for t in threads:
         t.join()
     assert not bad
+
+
+# Keys `depth` binades below a dominant one, all alike, so that the rounding of their probabilities does not average out.  A
+# stored probability ends 2^-17 below the reference maximum (half of that is the largest error), the output is bf16.
+@pytest.mark.parametrize("heads", [16, 32, 64, 128])
+@pytest.mark.parametrize("depth", [10, 12, 15])
+@pytest.mark.parametrize("at", [0, 3000])
+def test_coherent_tail_far_below_the_maximum(pkg, heads, depth, at):
+    n = 4097
+    g = torch.Generator().manual_seed(depth)
+    q = torch.zeros(1, heads, 576)
+    q[..., 0] = 4.0
+    kv = 1.0 + 0.25 * torch.randn(n, 576, generator=g)
+    kv[:, 0], kv[:, 512:] = 0.0, 0.0
+    kv[at, 0], kv[at, 1:512] = depth * 0.6931 / 4.0, 0.1 * torch.randn(511, generator=g)
+    codes, scale = pkg.quantize_fp8(kv.bfloat16().cuda())
+    qc, qs = pkg.quantize_q_fp8(q.bfloat16().cuda())
+    K = codes.reshape(n, 576).float().double() * scale.double()
+    want = torch.softmax(qc[0].float().double() * qs.double() @ K.T, -1) @ K[:, :512]
+    ip = torch.tensor([0, n], dtype=torch.int32, device="cuda")
+    for max_ctas in (1, 0):
+        got = pkg.mla_decode(qc, qs, "fp8", (codes, scale), ip, sm_scale=1.0, impl="tcgen05", max_ctas=max_ctas)[0].double()
+        assert float((got - want).norm() / want.norm()) <= 2.0 ** (depth - 18) + 2.0 ** -8
