@@ -56,10 +56,12 @@ class PeerMergeArgs(ctypes.Structure):
 
 APPEND_WRITE_STATUS = 1
 PEER_HANDLE_BYTES = 64
+GRAPH_WORDS = 256
 
 EXPORTS = ("b200_mla_version", "b200_mla_last_error", "b200_mla_workspace_bytes", "b200_mla_decode",
            "b200_mla_combine", "b200_mla_quantize_fp8", "b200_mla_q_amax", "b200_mla_set_stage1_events",
-           "b200_mla_decode_static", "b200_mla_read_status", "b200_mla_reset_status", "b200_mla_kv_append",
+           "b200_mla_decode_static", "b200_mla_read_status", "b200_mla_reset_status", "b200_mla_graph_workspace",
+           "b200_mla_graph_status", "b200_mla_kv_append",
            "b200_mla_peer_exchange_bytes", "b200_mla_peer_partial_offset", "b200_mla_peer_alloc", "b200_mla_peer_open",
            "b200_mla_peer_close", "b200_mla_peer_free", "b200_mla_peer_merge")
 STATUS_TIMEOUT, STATUS_BAD_PAGE = 1, 2
@@ -89,6 +91,10 @@ def _load() -> ctypes.CDLL:
     lib.b200_mla_read_status.argtypes = [_vp, _vp, _vp]
     lib.b200_mla_reset_status.restype = _i32
     lib.b200_mla_reset_status.argtypes = [_vp, _vp]
+    lib.b200_mla_graph_workspace.restype = _i32
+    lib.b200_mla_graph_workspace.argtypes = [_vp, _i32, _vp]
+    lib.b200_mla_graph_status.restype = _i32
+    lib.b200_mla_graph_status.argtypes = [_i32, _vp, _vp]
     lib.b200_mla_kv_append.restype = _i32
     lib.b200_mla_kv_append.argtypes = [ctypes.POINTER(KvAppendArgs), _vp]
     lib.b200_mla_peer_exchange_bytes.restype = _i64

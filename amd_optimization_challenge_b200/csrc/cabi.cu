@@ -216,6 +216,15 @@ int32_t b200_mla_decode(const b200_mla_decode_args* a, void* stream_) {
 // Scratch of the allocation-free entry point: lives in the library image, one copy per GPU.
 static __device__ __align__(256) unsigned char g_static_workspace[B200_MLA_STATIC_WORKSPACE_BYTES];
 
+// Status words of workspaces that live in CUDA graphs, and the kernel that makes such a workspace's header: all zero but for
+// the address of its word here.
+static __device__ int g_graph_status[B200_MLA_GRAPH_WORDS];
+static __global__ void graph_header_kernel(int* header, int word) {
+    const unsigned long long forward = reinterpret_cast<unsigned long long>(g_graph_status + word);
+    const int i = (int)threadIdx.x;
+    header[i] = i == ST_FORWARD ? (int)(forward & 0xffffffffu) : i == ST_FORWARD + 1 ? (int)(forward >> 32) : 0;
+}
+
 // Device address of the built-in scratch on the current device.  In host code the array's name is
 // only a handle; its device address is looked up once per device, with that device current.
 static int static_workspace_ptr(void** out) {
@@ -275,6 +284,23 @@ int32_t b200_mla_reset_status(void* workspace, void* stream) {
     }
     cudaError_t e = cudaMemsetAsync(workspace, 0, 256, (cudaStream_t)stream);
     if (e != cudaSuccess) return fail(B200_MLA_ERR_CUDA, "status reset failed: %s", cudaGetErrorString(e));
+    return B200_MLA_OK;
+}
+
+int32_t b200_mla_graph_workspace(void* workspace, int32_t word, void* stream) {
+    if (!workspace || ((uintptr_t)workspace & 255)) return fail(B200_MLA_ERR_INVALID_ARG, "workspace must be non-NULL and 256-byte aligned");
+    if (word < 0 || word >= B200_MLA_GRAPH_WORDS) return fail(B200_MLA_ERR_INVALID_ARG, "word %d outside [0, %d)", word, B200_MLA_GRAPH_WORDS);
+    graph_header_kernel<<<1, 64, 0, (cudaStream_t)stream>>>((int*)workspace, word);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(B200_MLA_ERR_CUDA, "workspace header launch failed: %s", cudaGetErrorString(e));
+    return B200_MLA_OK;
+}
+
+int32_t b200_mla_graph_status(int32_t word, int32_t* out, void* stream) {
+    if (!out) return fail(B200_MLA_ERR_INVALID_ARG, "out is NULL");
+    if (word < 0 || word >= B200_MLA_GRAPH_WORDS) return fail(B200_MLA_ERR_INVALID_ARG, "word %d outside [0, %d)", word, B200_MLA_GRAPH_WORDS);
+    cudaError_t e = cudaMemcpyFromSymbolAsync(out, g_graph_status, sizeof(int32_t), word * sizeof(int), cudaMemcpyDefault, (cudaStream_t)stream);
+    if (e != cudaSuccess) return fail(B200_MLA_ERR_CUDA, "status copy failed: %s", cudaGetErrorString(e));
     return B200_MLA_OK;
 }
 

@@ -39,9 +39,10 @@ inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, unsigned int
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Words of the 256-byte workspace header behind the status word, for launches whose CTAs work together.  They are zero
-// between launches: the last CTA to leave resets them.
-enum { SYNC_AMAX = 16, SYNC_AMAX_COUNT = 17, SYNC_PREFIX = 18, SYNC_ARRIVE = 32, SYNC_EXIT = 48 };
+// Words of the 256-byte workspace header behind the status word.  ST_FORWARD: address (two words) of a second status word that
+// receives the same bits, 0 if there is none.  SYNC_*: for launches whose CTAs work together; they are zero between launches:
+// the last CTA to leave resets them.
+enum { ST_FORWARD = 2, SYNC_AMAX = 16, SYNC_AMAX_COUNT = 17, SYNC_PREFIX = 18, SYNC_ARRIVE = 32, SYNC_EXIT = 48 };
 
 struct MlaParams {
     int batch, heads, q_len, rows;      // rows = q_len * heads (query rows per sequence)
@@ -240,6 +241,12 @@ __device__ __forceinline__ int off_in_page(const MlaParams& p, int pos) { return
 // two steps ahead of their use, and touching the value early would wait for that load (measured: 10-25 % of a call).
 __device__ __forceinline__ unsigned int clamp_slot(const MlaParams& p, int s) { return min((unsigned int)s, p.last_slot); }
 
+__device__ __forceinline__ void report_status(int* status, int bits) {
+    atomicOr(status, bits);
+    int* forward = *reinterpret_cast<int* const*>(status + ST_FORWARD);
+    if (forward) atomicOr(forward, bits);
+}
+
 // Page ids of the tiles [t_begin, t_end) a stage-1 CTA owns: sets ST_BAD_PAGE if one of them names a page outside
 // the cache planes (or, without a page table, if a token range reaches beyond them).  Called by `nthreads` threads
 // (tid = 0 .. nthreads - 1) that have nothing else to do at the time; `tile` = tokens per tile.  Inlined: a call would
@@ -265,7 +272,7 @@ __device__ __forceinline__ void check_span_pages(const MlaParams& p, const int* 
         }
         t = t1;
     }
-    if (bad) atomicOr(p.status, (int)ST_BAD_PAGE);
+    if (bad) report_status(p.status, ST_BAD_PAGE);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -863,7 +863,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                     advance(g, k);
                 }
                 cp_async_wait_all();
-                if (bad) atomicOr(p.status, (int)ST_BAD_PAGE);
+                if (bad) report_status(p.status, ST_BAD_PAGE);
             } else {
                 // Block-scaled cache: convert.  The auxiliary warps bring the units into the landing buffers, in rounds; a landed unit
                 // moves into registers, its buffer goes back at once, and the e4m3 operand bytes go to the stage.
@@ -1072,7 +1072,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                 }
             }
             cp_async_wait_all();
-            if (bad) atomicOr(p.status, (int)ST_BAD_PAGE);
+            if (bad) report_status(p.status, ST_BAD_PAGE);
         }
     }
 
@@ -1114,7 +1114,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
             p.status[SYNC_AMAX] = 0; p.status[SYNC_AMAX_COUNT] = 0; p.status[SYNC_PREFIX] = 0; p.status[SYNC_ARRIVE] = 0; p.status[SYNC_EXIT] = 0;
         }
     }
-    if (tid == 0 && ms.abort_flag) atomicOr(p.status, (int)ST_TIMEOUT);
+    if (tid == 0 && ms.abort_flag) report_status(p.status, ST_TIMEOUT);
 }
 
 }  // namespace sm100

@@ -257,6 +257,18 @@ int32_t b200_mla_read_status(const void *workspace, int32_t *out, void *stream);
 int32_t b200_mla_reset_status(void *workspace, void *stream);
 
 /*
+ * A workspace that lives in a CUDA graph (no counterpart in the reference, which captures nothing): its memory may belong to
+ * the graph and be gone, or used for something else, when the graph is.  b200_mla_graph_workspace takes the place of
+ * b200_mla_reset_status for it, once per capture, ahead of the first decode that uses it: every replay then starts from a clean
+ * header, and status bits also go to word `word` (0 .. B200_MLA_GRAPH_WORDS - 1) of an array that the library keeps on each
+ * device until the process exits.  b200_mla_graph_status enqueues the copy of that word into `out`, as b200_mla_read_status
+ * does; call it outside a capture.  A workspace of a graph must not be used outside it, nor by two graphs.
+ */
+#define B200_MLA_GRAPH_WORDS 256
+int32_t b200_mla_graph_workspace(void *workspace, int32_t word, void *stream);
+int32_t b200_mla_graph_status(int32_t word, int32_t *out, void *stream);
+
+/*
  * Profiling aid (no counterpart in the reference, whose harness times whole calls, eval.py:225-261):
  * while both events (cudaEvent_t) are non-NULL, every b200_mla_decode issued by the calling thread
  * records `start` before and `stop` after its stage-1 kernel on the call's stream.  Pass NULLs to

@@ -232,3 +232,73 @@ def test_coherent_tail_far_below_the_maximum(pkg, heads, depth, at):
     for max_ctas in (1, 0):
         got = pkg.mla_decode(qc, qs, "fp8", (codes, scale), ip, sm_scale=1.0, impl="tcgen05", max_ctas=max_ctas)[0].double()
         assert float((got - want).norm() / want.norm()) <= 2.0 ** (depth - 18) + 2.0 ** -8
+
+
+def _captured(pkg, data, n=1, stream=None):
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        outs = [pkg.custom_kernel(data) for _ in range(n)]
+    return graph, outs
+
+
+@pytest.mark.parametrize("kv_format,q_format,heads", [("fp8", "fp8", 16), ("mxfp4", "bf16", 32), ("hybrid", "fp8", 64)])
+def test_captures_with_and_without_an_earlier_call(pkg, kv_format, q_format, heads):
+    """A graph's scratch is its own: the second capture is replayed first, calls on the capturing stream come in between."""
+    lens = [700, 33, 1900, 0, 260]                               # a shape that no other test uses: no scratch from an earlier call
+    data = pkg.generate_input(5, 1, 1900, seed=heads, kv_lens=lens, shuffle_pages=True, num_heads=heads, formats=(kv_format,))
+    data = (*data[:4], dict(data[4], kv_format=kv_format, q_format=q_format))
+    want = oracle_for_data(data, kv_format, q_format)
+    s = torch.cuda.Stream()
+    g1, o1 = _captured(pkg, data, 2, s)
+    g2, o2 = _captured(pkg, data, 1, s)
+    with torch.cuda.stream(s):
+        for _ in range(2):
+            g2.replay()
+            assert_close(o2[0], want, tight=1.5e-2)
+            eager = pkg.custom_kernel(data)
+            assert_close(eager, want, tight=1.5e-2)
+        g3, o3 = _captured(pkg, data, 1, s)
+        del g2
+        for g, o in ((g3, o3), (g1, o1), (g3, o3)):
+            [t.zero_() for t in o]
+            g.replay()
+            assert all(torch.equal(t, eager) for t in o)
+    from amd_optimization_challenge_b200 import submission
+    assert not submission._graph_pinned                          # the scratch came from the graphs' own pool
+
+
+def test_replays_beside_calls_and_other_graphs_of_one_shape(pkg):
+    lens = [3000, 17, 900, 64]
+    sets = [pkg.generate_input(4, 1, 3000, seed=s, kv_lens=lens, shuffle_pages=True, formats=("fp8",)) for s in range(3)]
+    sets = [(*d[:4], dict(d[4], kv_format="fp8", q_format="fp8")) for d in sets]
+    want = [pkg.custom_kernel(d) for d in sets]
+    graphs = [_captured(pkg, d, 20) for d in sets[:2]]
+    streams = [torch.cuda.Stream() for _ in sets]
+    torch.cuda.synchronize()
+    eager = []
+    for _ in range(5):
+        for (g, _outs), s in zip(graphs, streams):
+            with torch.cuda.stream(s):
+                g.replay()
+        with torch.cuda.stream(streams[2]):
+            eager += [pkg.custom_kernel(sets[2]) for _ in range(20)]
+    torch.cuda.synchronize()
+    for (_g, outs), w in zip(graphs, want):
+        assert all(torch.equal(t, w) for t in outs)
+    assert all(torch.equal(t, want[2]) for t in eager)
+
+
+def test_status_of_replays_reaches_read_status(pkg):
+    from amd_optimization_challenge_b200 import _cabi, submission
+    lens = [40, 41, 42, 43, 44, 45]                              # this test's own shape: its status word is sticky
+    data = pkg.generate_input(6, 2, 45, seed=1, kv_lens=lens, shuffle_pages=True, formats=("mxfp4",))
+    data = (*data[:4], dict(data[4], kv_format="mxfp4", q_format="bf16"))
+    graph, outs = _captured(pkg, data)
+    graph.replay()
+    assert submission.read_status(outs[0].device, 6, 16, 2) == 0
+    data[4]["kv_indices"][100] = 1 << 20                         # outside the cache: reported, read as another row
+    graph.replay()
+    data[4]["kv_indices"][100] = 0
+    graph.replay()
+    assert submission.read_status(outs[0].device, 6, 16, 2) == _cabi.STATUS_BAD_PAGE
+    assert submission.read_status(outs[0].device, 6, 16, 1) == 0
