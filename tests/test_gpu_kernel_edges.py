@@ -302,3 +302,65 @@ def test_status_of_replays_reaches_read_status(pkg):
     graph.replay()
     assert submission.read_status(outs[0].device, 6, 16, 2) == _cabi.STATUS_BAD_PAGE
     assert submission.read_status(outs[0].device, 6, 16, 1) == 0
+
+
+@pytest.mark.parametrize("what", ["q", "plane", "scales", "kv_indptr", "kv_indices", "num_slots"])
+def test_repeated_calls_notice_tensors_changed_in_place(pkg, what):
+    """The same objects with other storage, sizes or strides.  (The old storage stays alive here.)"""
+    lens = [300, 40, 7]
+    data = pkg.generate_input(3, 1, 300, seed=3, kv_lens=lens, shuffle_pages=True, formats=("mxfp4",))
+    data = (*data[:4], dict(data[4], kv_format="mxfp4", q_format="bf16"))
+    other = pkg.generate_input(3, 1, 300, seed=4, kv_lens=lens, shuffle_pages=True, formats=("mxfp4",))
+    (codes, scales), table = data[1]["mxfp4"], data[4]["kv_indices"]
+    direct = lambda: pkg.mla_decode(data[0], None, "mxfp4", (codes, scales), data[3], sm_scale=data[4]["sm_scale"], kv_indices=table,
+                                    total_kv_hint=sum(lens))
+    check = lambda: [assert_close(o, oracle_for_data(data, "mxfp4", "bf16"), tight=1.5e-2) for o in (pkg.custom_kernel(data), direct())]
+    for _ in range(2):
+        check()
+    keep = [t.clone() for t in (data[0], codes, scales, data[3], table)], [t.detach() for t in (data[0], codes, scales, data[3], table)]
+    if what == "q":
+        data[0].data = other[0]
+    elif what == "plane":
+        codes.data = other[1]["mxfp4"][0]
+    elif what == "scales":                                       # the same rows behind another stride
+        wide = torch.zeros(scales.shape[0], 64, dtype=torch.uint8, device="cuda")
+        wide[:, :18] = scales[:, :18]
+        scales.data = wide
+    elif what == "kv_indptr":
+        data[3].data = torch.tensor([0, 200, 201, 300], dtype=torch.int32, device="cuda")
+    elif what == "kv_indices":
+        table.data = other[4]["kv_indices"]
+    else:                                                        # fewer rows at the same address: ids beyond them are not read
+        n = codes.shape[0] - 8
+        inside = table.clamp(max=n - 1)
+        codes.data = codes[:n]
+        rows = table.clone()
+        assert int((rows >= n).sum()) > 0
+        out = pkg.custom_kernel(data)
+        table.copy_(inside)
+        assert torch.equal(out, pkg.custom_kernel(data))         # read as the last row
+        from amd_optimization_challenge_b200 import _cabi, submission
+        assert submission.read_status(out.device, 3, 16, 1) == _cabi.STATUS_BAD_PAGE
+        ws = submission._workspace(out.device, 3, 16, 1)
+        _cabi.check(_cabi.lib.b200_mla_reset_status(ws.data_ptr(), torch.cuda.current_stream().cuda_stream), "reset")
+        return
+    for _ in range(2):
+        check()
+    del keep
+
+
+def test_append_notices_planes_changed_in_place(pkg):
+    g = torch.Generator().manual_seed(8)
+    rows, scale = torch.randn(40, 576, generator=g).bfloat16().cuda(), torch.full((1,), 0.01, device="cuda")
+    store = torch.zeros(100, 576, dtype=torch.uint8, device="cuda")
+    plane = store[:50]
+    for _ in range(2):
+        pkg.kv_append(rows, "fp8", (plane, scale))
+    want = store[:40].clone()
+    store.zero_()
+    plane.as_strided_((50, 576), (1152, 1))                      # every other row of the same memory
+    assert int(pkg.kv_append(rows, "fp8", (plane, scale))) == 0
+    assert torch.equal(store[:80:2], want) and int(store[1::2].max()) == 0
+    plane.as_strided_((39, 576), (1152, 1))                      # a row too few
+    with pytest.raises(RuntimeError, match="do not fit"):
+        pkg.kv_append(rows, "fp8", (plane, scale))

@@ -48,3 +48,19 @@ def test_generator_device_default_is_cpu_and_seeded():
     a = pkg.generate_input(2, 1, 8, seed=3, formats=("fp8",), device="cpu")
     b = pkg.generate_input(2, 1, 8, seed=3, formats=("fp8",), device="cpu", generator_device="cpu")
     assert torch.equal(a[0], b[0]) and torch.equal(a[1]["fp8"][0].view(torch.uint8), b[1]["fp8"][0].view(torch.uint8))
+
+
+def test_signature_sees_storage_and_shape():
+    from amd_optimization_challenge_b200._host import signature
+    t = torch.zeros(6, 4)
+    old = t.detach()
+    first = signature([t, None])
+    assert first == signature((t, None)) != signature((t,))
+    for change in (lambda: t.as_strided_((6, 2), (4, 1)), lambda: t.as_strided_((6, 2), (2, 1)), lambda: t.resize_(5, 2),
+                   lambda: setattr(t, "data", torch.zeros(5, 2)), lambda: setattr(t, "data", torch.zeros(5, 2, dtype=torch.int32))):
+        before = signature([t])
+        change()
+        assert signature([t]) != before
+    assert signature([old, None]) == first
+    with pytest.raises(RuntimeError):
+        signature([torch.zeros(3, 3).to_sparse()])
