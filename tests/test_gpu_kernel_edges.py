@@ -364,3 +364,33 @@ def test_append_notices_planes_changed_in_place(pkg):
     plane.as_strided_((39, 576), (1152, 1))                      # a row too few
     with pytest.raises(RuntimeError, match="do not fit"):
         pkg.kv_append(rows, "fp8", (plane, scale))
+
+
+@pytest.mark.parametrize("kv_format", ["fp8", "mxfp4", "hybrid"])
+def test_append_to_planes_with_gaps_between_pages(pkg, kv_format):
+    """Rows that no single stride describes, again and again: they reach the planes, and nothing else is written."""
+    from amd_optimization_challenge_b200 import inputs
+    g = torch.Generator().manual_seed(3)
+    pages, used, room = 5, 24, 32
+    rows = torch.randn(pages * used, 1, 576, generator=g).bfloat16()
+    quant = {"fp8": inputs.quantize_fp8, "mxfp4": inputs.quantize_mxfp4, "hybrid": inputs.quantize_hybrid}[kv_format](rows)
+    want = [t.view(torch.uint8).reshape(pages * used, -1) for t in quant if t.dim() > 1]
+    gapped = lambda w: torch.full((pages, room, w.shape[1]), 0xEE, dtype=torch.uint8, device="cuda")
+    kv, stores = [], []
+    for t in quant:
+        if t.dim() <= 1:
+            kv.append(t.cuda())
+        elif t is quant[1]:                                      # E8M0 rows: two-dimensional by contract
+            kv.append(torch.full((pages * used, t.shape[-1]), 0xEE, dtype=torch.uint8, device="cuda"))
+        else:
+            stores.append(gapped(t.view(torch.uint8).reshape(pages * used, -1)))
+            kv.append(stores[-1][:, :used])
+    for _ in range(3):
+        for t in kv:
+            if t.dtype == torch.uint8:
+                t.fill_(0xEE)
+        other = [torch.zeros_like(s) for s in stores]            # takes the place of freed copies
+        assert int(pkg.kv_append(rows.cuda(), kv_format, tuple(kv))) == 0
+        got = [t.reshape(pages * used, -1).cpu() for t in kv if t.dtype == torch.uint8]
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        assert all(bool((s[:, used:] == 0xEE).all()) for s in stores) and not any(bool(t.any()) for t in other)
