@@ -117,7 +117,7 @@ int32_t b200_mla_decode(const b200_mla_decode_args* a, void* stream_) {
         return fail(B200_MLA_ERR_INVALID_ARG, "bad kv_format %d", a->kv_format);
     if (!a->q || !a->kv_codes || !a->kv_indptr) return fail(B200_MLA_ERR_INVALID_ARG, "q, kv_codes and kv_indptr are required");
     const bool quant = a->q_format == B200_MLA_Q_BF16_QUANT_E4M3;
-    if (quant && (a->q_head_stride != QK_DIM || a->q_row_stride != (int64_t)a->heads * QK_DIM))
+    if (quant && (a->q_head_stride != QK_DIM || ((int64_t)a->batch * a->q_len > 1 && a->q_row_stride != (int64_t)a->heads * QK_DIM)))
         return fail(B200_MLA_ERR_INVALID_ARG, "a Q that the call quantises must be dense");
     if (a->q_format != B200_MLA_Q_BF16 && !quant && !a->q_scale)
         return fail(B200_MLA_ERR_INVALID_ARG, "q_scale is required for e4m3 Q (the scale, or the amax partials when Q is cast on load)");

@@ -394,3 +394,16 @@ def test_append_to_planes_with_gaps_between_pages(pkg, kv_format):
         got = [t.reshape(pages * used, -1).cpu() for t in kv if t.dtype == torch.uint8]
         assert all(torch.equal(a, b) for a, b in zip(got, want))
         assert all(bool((s[:, used:] == 0xEE).all()) for s in stores) and not any(bool(t.any()) for t in other)
+
+
+@pytest.mark.parametrize("q_format", ["fp8", "bf16"])
+@pytest.mark.parametrize("impl", ["tcgen05", "generic"])
+def test_one_query_row_that_is_a_slice(pkg, impl, q_format):
+    """One query token, its heads a slice of more: contiguous to torch, with the stride of the wider tensor."""
+    data = pkg.generate_input(1, 1, 300, seed=6, formats=("fp8",))
+    wide = torch.cat((data[0], 3 * data[0], data[0][:, :5]), 1)
+    part = (wide[:, :16], *data[1:])
+    assert part[0].is_contiguous() and part[0].stride(0) == 37 * 576
+    want = oracle_for_data(data, "fp8", q_format)
+    for _ in range(2):
+        assert_close(_run(pkg, part, "fp8", q_format, impl=impl), want, tight=1.5e-2)
