@@ -1,12 +1,18 @@
 """Host-side argument checks of the Python mirror (no GPU needed): what the kernels would misread on
 the device - a page table of the wrong dtype, on the wrong device or strided - is refused before any
 launch, because a bad index on the GPU is an out-of-bounds read rather than an exception."""
+import os
+import subprocess
+import sys
+import textwrap
+
 import pytest
 import torch
 
 from amd_optimization_challenge_b200 import submission as sub
 
 CPU = torch.device("cpu")
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def test_index_tensor_checks():
@@ -64,3 +70,26 @@ def test_signature_sees_storage_and_shape():
     assert signature([old, None]) == first
     with pytest.raises(RuntimeError):
         signature([torch.zeros(3, 3).to_sparse()])
+
+
+def test_append_of_a_tensor_without_strides_raises():
+    """Tensors that answer questions about themselves in Python, and may refuse: an exception, not the end of the process."""
+    code = textwrap.dedent("""
+        import torch
+        from amd_optimization_challenge_b200 import submission as sub
+        class T(torch.Tensor):
+            @staticmethod
+            def __new__(cls, shape, dtype):
+                return torch.Tensor._make_wrapper_subclass(cls, shape, dtype=dtype, device="cuda", dispatch_sizes_strides_policy="strides")
+            @classmethod
+            def __torch_dispatch__(cls, f, types, args=(), kwargs=None):
+                raise NotImplementedError("no strides")
+        planes = T((9, 576), torch.uint8), T((1,), torch.float32)
+        for call in (lambda: sub.kv_append(T((4, 576), torch.bfloat16), "fp8", planes), lambda: sub._host.signature(planes)):
+            try:
+                call()
+            except NotImplementedError as e:
+                print("RAISED", e)
+    """)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=ROOT)
+    assert r.returncode == 0 and r.stdout.count("RAISED no strides") == 2, r.stdout + r.stderr
