@@ -93,3 +93,9 @@ def test_append_of_a_tensor_without_strides_raises():
     """)
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=ROOT)
     assert r.returncode == 0 and r.stdout.count("RAISED no strides") == 2, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("base", [3.0, torch.tensor(3), 1 << 70])
+def test_append_takes_what_int_takes_as_base_slot(base):
+    with pytest.raises(ValueError, match="CUDA"):                # the rows are refused, not the slot
+        sub.kv_append(torch.zeros(2, 576, dtype=torch.bfloat16), "fp8", (torch.zeros(9, 576, dtype=torch.uint8), torch.ones(1)), base_slot=base)
