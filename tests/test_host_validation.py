@@ -5,6 +5,7 @@ import os
 import subprocess
 import sys
 import textwrap
+import threading
 
 import pytest
 import torch
@@ -99,3 +100,47 @@ def test_append_of_a_tensor_without_strides_raises():
 def test_append_takes_what_int_takes_as_base_slot(base):
     with pytest.raises(ValueError, match="CUDA"):                # the rows are refused, not the slot
         sub.kv_append(torch.zeros(2, 576, dtype=torch.bfloat16), "fp8", (torch.zeros(9, 576, dtype=torch.uint8), torch.ones(1)), base_slot=base)
+
+
+def test_remembering_replaces_and_evicts():
+    cache = {i: i for i in range(4)}
+    sub._remember(cache, 2, "new", limit=4)                      # a key that is there: nothing else leaves, and it is the newest
+    assert cache == {0: 0, 1: 1, 3: 3, 2: "new"}
+    for i in (7, 8, 9):
+        sub._remember(cache, i, i, limit=4)
+    assert list(cache) == [2, 7, 8, 9]
+
+
+def test_plan_caches_with_threads(monkeypatch):
+    """Calls of one tensor set with changing numbers, from threads that make each other's plans stale."""
+    class Q:                                                     # what mla_decode looks at before it comes to the plan
+        is_cuda = True
+    q, ip = Q(), Q()
+    plans = {}
+    monkeypatch.setattr(sub, "_decode_plans", plans)
+
+    class Stale:
+        signature = refs = ()
+        @property
+        def scalars(self):                                       # another thread takes the plan out while this one looks at it
+            plans.clear()
+            return ()
+    plans[(id(q), id(ip), id(None), "fp8", False)] = Stale()
+    with pytest.raises(AttributeError):                          # past the plans, on to the arguments
+        sub.mla_decode(q, None, "fp8", (), ip, sm_scale=1.0)
+    cache, errors = {}, []
+
+    def work(n):
+        try:
+            for i in range(20000):
+                sub._remember(cache, (n, i % 50), i, limit=8)
+                cache.pop((1 - n, i % 50), None)
+        except Exception as e:
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=(n,)) for n in (0, 1)]
+    old = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    sys.setswitchinterval(old)
+    assert not errors
