@@ -10,9 +10,9 @@
 //     mxfp4-mm/submission_v3_self_contained.py:19-72; reference.py:88-113), two codes per byte, even element
 //     in the low nibble.
 //   * hybrid: dims 0..511 as MXFP4 (16 blocks), dims 512..575 as e4m3 with the per-tensor rope scale.
-// One thread quantises eight elements (16 bytes in; 8 or 4 bytes out), so that neighbouring lanes read and write
-// neighbouring bytes; the four lanes of a 32-element block share its exponent by two shuffles.  HBM bound from a few
-// thousand rows on, launch and load latency below.
+// One thread quantises eight elements, or sixteen of an e4m3 row (16 bytes a load; 16 or 4 a store), so that neighbouring lanes
+// read and write neighbouring bytes; the four lanes of a 32-element block share its exponent by two shuffles.  HBM bound from
+// some ten thousand rows on, launch and load latency below.
 #include "mla_common.cuh"
 #include "sm100_ptx.cuh"
 
@@ -25,7 +25,6 @@ using namespace sm100;
 struct AppendParams {
     const __nv_bfloat16* src; long long n; long long src_stride;   // elements between rows
     const int* slots; long long base_slot; long long num_slots;
-    int kv_format;
     uint8_t* codes; long long codes_stride;
     uint8_t* bs; long long bs_stride;
     uint8_t* rope; long long rope_stride;
@@ -34,27 +33,25 @@ struct AppendParams {
     int write_status;                                               // the last block looks the slots over and writes *bad, 0 or 1
 };
 
-constexpr int CHUNKS = QK_DIM / 8;                                  // 72 threads share a row
-constexpr int STEP = 4;                                             // rows a block covers at a time
-constexpr int DEPTH = 2;                                            // rows a thread has in flight
+constexpr int THREADS = 288;
 constexpr int RESIDENT = 7;                                         // blocks on an SM
+constexpr int vectors(int kv_format) { return kv_format == KV_E4M3 ? 2 : 1; }                   // of eight elements per thread
+constexpr int block_rows(int kv_format) { return THREADS * 8 * vectors(kv_format) / QK_DIM; }   // rows a block covers at a time
 
 __device__ __forceinline__ f32x2 widen(uint32_t w) { return pk2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 
 // Eight bf16 values -> their e4m3 codes, the codes of q_cast_e4m3x8 (mla_common.cuh) for every input: two values per
-// instruction, and the quotients that need its special cases (infinite or NaN) are left to it.  r = RN(1 / scale).
-__device__ __forceinline__ uint2 cast_e4m3x8(const uint4& v, float scale, float r) {
+// instruction, and vectors that may need its special cases (infinite or NaN quotients) are left to it: those with a value whose
+// magnitude bits reach `general` (general_from).  r = RN(1 / scale).
+__device__ __forceinline__ uint2 cast_e4m3x8(const uint4& v, float scale, float r, unsigned int general) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     const f32x2 s2 = pk2(-scale, -scale), r2 = pk2(r, r);
-    uint32_t c[4];
-    float top = 0.0f;
+    uint32_t c[4], m = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
+        m = __vmaxu2(m, w[k] & 0x7fff7fffu);
         const f32x2 x = widen(w[k]), t = mul2(x, r2);
-        float t0, t1, y0, y1;
-        unpk2(t, t0, t1);
-        asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(t0)));
-        asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(t1)));
+        float y0, y1;
         unpk2(fma2(fma2(t, s2, x), r2, t), y0, y1);
         uint32_t h;
         asm("cvt.rn.bf16x2.f32 %0, %2, %1;" : "=r"(h) : "f"(y0), "f"(y1));
@@ -64,8 +61,13 @@ __device__ __forceinline__ uint2 cast_e4m3x8(const uint4& v, float scale, float 
         asm("cvt.rn.satfinite.e4m3x2.f32 %0, %2, %1;" : "=h"(q) : "f"(y0), "f"(y1));
         c[k] = q;
     }
-    if (!(top <= 3.0e38f)) return q_cast_e4m3x8(v, scale);
+    if (max(m & 0xffffu, m >> 16) >= general) return q_cast_e4m3x8(v, scale);
     return make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16));
+}
+// Magnitude bits (exponent field f) below which |x r| < 2^127 and finite: |x| < 2^(f - 126), |r| < 2^(e - 126), e its exponent field.
+__device__ __forceinline__ unsigned int general_from(float r) {
+    const int e = (int)((__float_as_uint(r) >> 23) & 0xffu);
+    return e == 255 ? 0u : (unsigned int)min(380 - e, 255) << 7;
 }
 
 // Eight bf16 values of a 32-element block whose other values are in the lanes of the same aligned group of four -> eight
@@ -111,66 +113,92 @@ __device__ __forceinline__ uint32_t quant_mxfp4x8(const uint4& v, uint8_t& scale
     return codes;
 }
 
-// A block covers STEP rows at a time and each thread holds up to DEPTH of its rows in flight.  16384 rows into an e4m3 cache
-// (28 MB moved): 7.7 us from one launch to the next, 10.2 us with a 32-element block (64 bytes in strides) per thread, 64-bit
-// divisions and the full launch gap.  Two rows in flight on seven resident blocks were the best of what was tried: 8.3 us with
-// two on five, 9.8 with four on five and 10.4 with four on seven (registers spill), 7.9 with one on seven.
-template <int KVFMT>
-__global__ void __launch_bounds__(STEP * CHUNKS, RESIDENT) kv_append_kernel(const AppendParams p) {
+// Instructions bound it next to HBM, so a thread keeps pointers and advances them, and an e4m3 thread has two vectors: 500000
+// rows into an e4m3 cache (864 MB moved) 158 us with listed slots and 146 without, 205 and 176 with one vector and 64-bit
+// products per row.  A block's first loads are issued before anything that waits for the scale.  Seven resident blocks, one step
+// in flight each: two steps spill registers (16384 rows, e4m3: 6.3 us from one launch to the next with one step, 7.9 with two).
+template <int KVFMT, bool LISTED>
+__global__ void __launch_bounds__(THREADS, RESIDENT) kv_append_kernel(const AppendParams p) {
     pdl_wait();
+    constexpr int VEC = vectors(KVFMT), CHUNKS = QK_DIM / 8 / VEC, STEP = block_rows(KVFMT);
     const int lead = p.write_status;
+    const unsigned int top = (unsigned int)min(p.num_slots, 1ll << 31);               // a negative slot is above it
     if ((int)blockIdx.x < lead) {
         // Slots are looked over once more by one block: *bad has to be 0 where all are good, and nobody zeroes it before.
-        const int n4 = p.slots && ((uintptr_t)p.slots & 15) == 0 ? (int)min(p.n / 4, 0x7fffffffll) : 0;
+        const int n4 = LISTED && ((uintptr_t)p.slots & 15) == 0 ? (int)min(p.n / 4, 0x7fffffffll) : 0;
         bool any = false;
-        const unsigned int top = (unsigned int)min(p.num_slots, 1ll << 31);           // a negative slot is above it
 #pragma unroll 8
-        for (int i = threadIdx.x; i < n4; i += STEP * CHUNKS) {
+        for (int i = threadIdx.x; i < n4; i += THREADS) {
             const int4 s = __ldg(reinterpret_cast<const int4*>(p.slots) + i);
             any |= max(max((unsigned int)s.x, (unsigned int)s.y), max((unsigned int)s.z, (unsigned int)s.w)) >= top;
         }
-        if (p.slots)
-            for (long long i = 4ll * n4 + threadIdx.x; i < p.n; i += STEP * CHUNKS) any |= (unsigned int)__ldg(p.slots + i) >= top;
+        if (LISTED)
+            for (long long i = 4ll * n4 + threadIdx.x; i < p.n; i += THREADS) any |= (unsigned int)__ldg(p.slots + i) >= top;
         any = __syncthreads_or(any);
         if (threadIdx.x == 0) *p.bad = any ? 1 : 0;
         return;
     }
-    const float scale = KVFMT != KV_MXFP4 ? __ldg(p.scale) : 1.0f, rscale = __frcp_rn(scale);
     const int sub = (int)threadIdx.x / CHUNKS, chunk = (int)threadIdx.x - sub * CHUNKS;
-    const long long hop = (long long)((int)gridDim.x - lead) * STEP;
-    for (long long row0 = (long long)((int)blockIdx.x - lead) * STEP; row0 < p.n; row0 += hop * DEPTH) {
-        uint4 v[DEPTH];
-        int listed[DEPTH];
+    const long long hop = (long long)((int)gridDim.x - lead) * STEP, row0 = (long long)((int)blockIdx.x - lead) * STEP;
+    const uint4* src = reinterpret_cast<const uint4*>(p.src + (row0 + sub) * p.src_stride) + chunk * VEC;
+    const long long src_hop = hop * p.src_stride / 8;
+    const int* list = p.slots + row0 + sub;
+    long long to = p.base_slot + row0 + sub;                                          // row of the cache, where no slots are listed
+    long long left = p.n - row0;                                                      // rows from the block's first one on
+    uint4 v[VEC];
+    unsigned int slot;
+    auto fetch = [&]() {
+        slot = 0xffffffffu;
 #pragma unroll
-        for (int i = 0; i < DEPTH; ++i) {
-            const long long row = row0 + sub + i * hop;
-            v[i] = make_uint4(0u, 0u, 0u, 0u);
-            listed[i] = 0;
-            if (row < p.n) {
-                if (p.slots) listed[i] = __ldg(p.slots + row);
-                v[i] = __ldg(reinterpret_cast<const uint4*>(p.src + row * p.src_stride) + chunk);
-            }
+        for (int k = 0; k < VEC; ++k) v[k] = make_uint4(0u, 0u, 0u, 0u);
+        if (sub < left) {
+            if (LISTED) slot = (unsigned int)__ldg(list);
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) v[k] = __ldg(src + k);
         }
-#pragma unroll
-        for (int i = 0; i < DEPTH; ++i) {
-            if (i > 0 && row0 + i * hop >= p.n) break;                            // the same for the whole block
-            const long long row = row0 + sub + i * hop, slot = p.slots ? (long long)listed[i] : p.base_slot + row;
-            const bool ok = row < p.n && slot >= 0 && slot < p.num_slots;         // nothing is written elsewhere
-            if (!ok && !p.write_status && row < p.n) *p.bad = 1;
-            if (KVFMT == KV_E4M3) {
-                if (ok) reinterpret_cast<uint2*>(p.codes + slot * p.codes_stride)[chunk] = cast_e4m3x8(v[i], scale, rscale);
-                continue;
+        src += src_hop;
+        list += hop;
+    };
+    const float scale = KVFMT != KV_MXFP4 ? __ldg(p.scale) : 1.0f;
+    fetch();
+    const float rscale = __frcp_rn(scale);
+    const unsigned int general = general_from(rscale);
+    for (;;) {                                                                        // the same number of steps for the whole block
+        const bool mine = sub < left, ok = LISTED ? slot < top : mine;                // nothing is written elsewhere
+        if (LISTED) {
+            if (mine && !ok && !p.write_status) *p.bad = 1;
+            to = (long long)slot;
+        }
+        if constexpr (KVFMT == KV_E4M3) {
+            static_assert(VEC == 2, "one 16-byte store");
+            if (ok) {
+                const uint2 a = cast_e4m3x8(v[0], scale, rscale, general), b = cast_e4m3x8(v[1], scale, rscale, general);
+                reinterpret_cast<uint4*>(p.codes + to * p.codes_stride)[chunk] = make_uint4(a.x, a.y, b.x, b.y);
             }
+        } else {
             uint8_t sb;
-            const uint32_t codes = quant_mxfp4x8(v[i], sb);
+            const uint32_t codes = quant_mxfp4x8(v[0], sb);
             if (KVFMT == KV_HYBRID && chunk >= V_DIM / 8) {
-                if (ok) reinterpret_cast<uint2*>(p.rope + slot * p.rope_stride)[chunk - V_DIM / 8] = cast_e4m3x8(v[i], scale, rscale);
+                if (ok) reinterpret_cast<uint2*>(p.rope + to * p.rope_stride)[chunk - V_DIM / 8] = cast_e4m3x8(v[0], scale, rscale, general);
             } else if (ok) {
-                reinterpret_cast<uint32_t*>(p.codes + slot * p.codes_stride)[chunk] = codes;
-                if ((chunk & 3) == 0) p.bs[slot * p.bs_stride + (chunk >> 2)] = sb;
+                reinterpret_cast<uint32_t*>(p.codes + to * p.codes_stride)[chunk] = codes;
+                if ((chunk & 3) == 0) p.bs[to * p.bs_stride + (chunk >> 2)] = sb;
             }
         }
+        left -= hop;
+        if (left <= 0) break;
+        to += hop;
+        fetch();
     }
+}
+
+// Up to eight steps per block of a single resident wave the blocks stay and loop (16384 rows, e4m3: 6.3 us, 7.8 with a wave
+// more); beyond that four waves even out what the blocks take (131072 rows: 38.4 us, 44.8 with one).
+template <int KVFMT>
+cudaError_t launch_format(const AppendParams& p, cudaStream_t stream) {
+    const long long wave = 148 * RESIDENT, steps = (p.n + block_rows(KVFMT) - 1) / block_rows(KVFMT), cap = steps <= 8 * wave ? wave : 4 * wave;
+    const unsigned int blocks = (unsigned int)(steps < cap ? steps : cap) + (unsigned int)p.write_status;
+    return launch_pdl(p.slots ? kv_append_kernel<KVFMT, true> : kv_append_kernel<KVFMT, false>, blocks, THREADS, stream, p);
 }
 
 }  // namespace
@@ -181,16 +209,13 @@ cudaError_t launch_kv_append(const void* src, long long n, long long src_stride,
                              bool write_status, cudaStream_t stream) {
     AppendParams p;
     p.src = (const __nv_bfloat16*)src; p.n = n; p.src_stride = src_stride;
-    p.slots = slots; p.base_slot = base_slot; p.num_slots = num_slots; p.kv_format = kv_format;
+    p.slots = slots; p.base_slot = base_slot; p.num_slots = num_slots;
     p.codes = (uint8_t*)codes; p.codes_stride = codes_stride;
     p.bs = (uint8_t*)bs; p.bs_stride = bs_stride;
     p.rope = (uint8_t*)rope; p.rope_stride = rope_stride;
     p.scale = scale; p.bad = bad; p.write_status = write_status ? 1 : 0;
-    const long long steps = (n + STEP - 1) / STEP, cap = 148 * RESIDENT;
-    const unsigned int blocks = (unsigned int)(steps < cap ? steps : cap) + (write_status ? 1u : 0u);
-    return launch_pdl(kv_format == KV_E4M3 ? kv_append_kernel<KV_E4M3> : kv_format == KV_MXFP4 ? kv_append_kernel<KV_MXFP4>
-                                                                                              : kv_append_kernel<KV_HYBRID>,
-                      blocks, STEP * CHUNKS, stream, p);
+    if (kv_format == KV_E4M3) return launch_format<KV_E4M3>(p, stream);
+    return kv_format == KV_MXFP4 ? launch_format<KV_MXFP4>(p, stream) : launch_format<KV_HYBRID>(p, stream);
 }
 
 }  // namespace b200mla

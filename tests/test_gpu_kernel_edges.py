@@ -407,3 +407,36 @@ def test_one_query_row_that_is_a_slice(pkg, impl, q_format):
     want = oracle_for_data(data, "fp8", q_format)
     for _ in range(2):
         assert_close(_run(pkg, part, "fp8", q_format, impl=impl), want, tight=1.5e-2)
+
+
+# Special values next to ordinary ones, in both vectors of a thread, and scales at which quotients overflow: the codes of the
+# division by the scale.
+@pytest.mark.parametrize("scale", [0.01, 1.0, 2.0 ** -100, 2.0 ** 100])
+def test_append_casts_special_values_as_the_division_does(pkg, scale):
+    g = torch.Generator().manual_seed(1)
+    rows = (torch.randn(37, 576, generator=g) * torch.exp2(torch.randint(-40, 40, (37, 576), generator=g).float())).bfloat16()
+    rows[3, 8], rows[4, 15], rows[5, 16] = float("inf"), float("-inf"), 3.0e38
+    rows[6, 1], rows[7, 9], rows[8, 575] = -3.0e38, float("nan"), -0.0
+    q = (rows.float() / torch.tensor(scale)).bfloat16().float()
+    want = q.clamp(-448.0, 448.0).to(torch.float8_e4m3fn).view(torch.uint8)
+    got = torch.zeros(37, 576, dtype=torch.uint8, device="cuda")
+    assert int(pkg.kv_append(rows.cuda(), "fp8", (got, torch.tensor([scale]).cuda()))) == 0
+    got, nan = got.cpu(), torch.isnan(q)
+    assert torch.equal(got[~nan], want[~nan]) and bool(((got[nan] & 0x7f) == 0x7f).all())
+
+
+# e4m3: 8 rows a block and step, 4 else; 1036 blocks stay for up to eight steps, then there are 4144
+@pytest.mark.parametrize("kv_format,n", [("fp8", 8 * 8288 - 1), ("fp8", 8 * 8288 + 1), ("mxfp4", 4 * 8288 + 1), ("hybrid", 4 * 8288 + 1), ("fp8", 200001)])
+def test_append_rows_around_the_wave_rule(pkg, kv_format, n):
+    from amd_optimization_challenge_b200 import inputs
+    few = torch.randn(997, 1, 576, generator=torch.Generator().manual_seed(n)).bfloat16()
+    quant = {"fp8": inputs.quantize_fp8, "mxfp4": inputs.quantize_mxfp4, "hybrid": inputs.quantize_hybrid}[kv_format](few)
+    pick = torch.arange(n, device="cuda") % 997
+    rows = few.cuda()[pick]
+    for slots in (None, torch.randperm(n, device="cuda").to(torch.int32)):
+        kv = tuple(torch.zeros(n, t.view(torch.uint8).reshape(997, -1).shape[1], dtype=torch.uint8, device="cuda") if t.dim() > 1 else t.cuda() for t in quant)
+        assert int(pkg.kv_append(rows, kv_format, kv, slots=slots)) == 0
+        at = slice(None) if slots is None else slots.long()
+        for plane, t in zip(kv, quant):
+            if t.dim() > 1:
+                assert torch.equal(plane[at], t.view(torch.uint8).reshape(997, -1).cuda()[pick])
