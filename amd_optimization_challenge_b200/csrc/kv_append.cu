@@ -125,15 +125,21 @@ __global__ void __launch_bounds__(THREADS, RESIDENT) kv_append_kernel(const Appe
     const unsigned int top = (unsigned int)min(p.num_slots, 1ll << 31);               // a negative slot is above it
     if ((int)blockIdx.x < lead) {
         // Slots are looked over once more by one block: *bad has to be 0 where all are good, and nobody zeroes it before.
-        const int n4 = LISTED && ((uintptr_t)p.slots & 15) == 0 ? (int)min(p.n / 4, 0x7fffffffll) : 0;
+        // Single ones up to a 16-byte boundary and after the last, four at a time between: a list that is a slice of a longer one
+        // starts anywhere (500000 rows, e4m3: 167 us one word at a time, 158 so).
         bool any = false;
+        if (LISTED) {
+            const int tid = (int)threadIdx.x, head = (int)min((long long)((0u - (unsigned int)(uintptr_t)p.slots) >> 2 & 3u), p.n);
+            const long long n4 = (p.n - head) >> 2, tail = head + 4 * n4;
+            const int4* s4 = reinterpret_cast<const int4*>(p.slots + head);
+            if (tid < head) any = (unsigned int)__ldg(p.slots + tid) >= top;
+            if (tail + tid < p.n) any |= (unsigned int)__ldg(p.slots + tail + tid) >= top;
 #pragma unroll 8
-        for (int i = threadIdx.x; i < n4; i += THREADS) {
-            const int4 s = __ldg(reinterpret_cast<const int4*>(p.slots) + i);
-            any |= max(max((unsigned int)s.x, (unsigned int)s.y), max((unsigned int)s.z, (unsigned int)s.w)) >= top;
+            for (long long i = tid; i < n4; i += THREADS) {
+                const int4 s = __ldg(s4 + i);
+                any |= max(max((unsigned int)s.x, (unsigned int)s.y), max((unsigned int)s.z, (unsigned int)s.w)) >= top;
+            }
         }
-        if (LISTED)
-            for (long long i = 4ll * n4 + threadIdx.x; i < p.n; i += THREADS) any |= (unsigned int)__ldg(p.slots + i) >= top;
         any = __syncthreads_or(any);
         if (threadIdx.x == 0) *p.bad = any ? 1 : 0;
         return;

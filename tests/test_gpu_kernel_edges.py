@@ -440,3 +440,21 @@ def test_append_rows_around_the_wave_rule(pkg, kv_format, n):
         for plane, t in zip(kv, quant):
             if t.dim() > 1:
                 assert torch.equal(plane[at], t.view(torch.uint8).reshape(997, -1).cuda()[pick])
+
+
+@pytest.mark.parametrize("off", [0, 1, 2, 3])
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 9, 1163])
+def test_append_reports_a_bad_slot_wherever_it_stands(pkg, n, off):
+    """The slots are looked over one by one up to a 16-byte boundary, then in fours, then one by one."""
+    rows = torch.zeros(n, 576, dtype=torch.bfloat16, device="cuda")
+    planes = torch.zeros(n, 288, dtype=torch.uint8, device="cuda"), torch.zeros(n, 18, dtype=torch.uint8, device="cuda")
+    around = torch.full((n + 8,), -7, dtype=torch.int32, device="cuda")              # what lies before and behind is not looked at
+    slots = around[off:off + n]
+    slots.copy_(torch.arange(n))
+    assert int(pkg.kv_append(rows, "mxfp4", planes, slots=slots)) == 0
+    for i in sorted({0, 1, 2, 3, 4, n // 2, n - 5, n - 4, n - 3, n - 2, n - 1} & set(range(n))):
+        for bad in (-1, n):
+            slots[i] = bad
+            assert int(pkg.kv_append(rows, "mxfp4", planes, slots=slots)) == 1
+        slots[i] = i
+    assert int(pkg.kv_append(rows, "mxfp4", planes, slots=slots)) == 0
