@@ -40,7 +40,7 @@ class KvAppendArgs(ctypes.Structure):
     """struct b200_mla_kv_append_args"""
     _fields_ = [
         ("rows_bf16", _vp), ("n", _i64), ("row_stride", _i64), ("slots", _vp), ("base_slot", _i64), ("num_slots", _i64),
-        ("kv_format", _i32), ("flags", _i32),
+        ("kv_format", _i32), ("reserved", _i32),
         ("kv_codes", _vp), ("kv_codes_stride", _i64), ("kv_block_scales", _vp), ("kv_block_scales_stride", _i64),
         ("kv_rope", _vp), ("kv_rope_stride", _i64), ("kv_scale", _vp), ("status", _vp),
     ]
@@ -54,7 +54,7 @@ class PeerMergeArgs(ctypes.Structure):
     ]
 
 
-APPEND_WRITE_STATUS = 1
+APPEND_WRITE_STATUS = 256
 PEER_HANDLE_BYTES = 64
 GRAPH_WORDS = 256
 

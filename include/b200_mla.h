@@ -186,9 +186,9 @@ int32_t b200_mla_quantize_fp8(const void *x_bf16, int64_t n, void *codes_out, fl
  * The per-tensor scale of an e4m3 cache / of a hybrid cache's rope dims is an input (device fp32[1]): rows added
  * later cannot change the scale of rows already stored.  A slot outside [0, num_slots) is not written and sets
  * *status (device int32, required with a slot list) to 1.  *status is not touched otherwise, so that it can collect
- * several calls; with B200_MLA_APPEND_WRITE_STATUS the call writes it, 0 or 1, and it needs no initialisation.
+ * several calls; with B200_MLA_APPEND_WRITE_STATUS added to kv_format the call writes it, 0 or 1, and it needs no initialisation.
  */
-#define B200_MLA_APPEND_WRITE_STATUS 1
+#define B200_MLA_APPEND_WRITE_STATUS 256
 typedef struct {
     const void *rows_bf16;    /* device bf16 [n, 576], 16-byte aligned */
     int64_t n;
@@ -196,8 +196,8 @@ typedef struct {
     const int32_t *slots;     /* device int32[n] destination slots, or NULL */
     int64_t base_slot;        /* first destination slot when slots is NULL */
     int64_t num_slots;        /* rows in the cache planes */
-    int32_t kv_format;        /* b200_mla_kv_format */
-    int32_t flags;            /* 0 or B200_MLA_APPEND_WRITE_STATUS */
+    int32_t kv_format;        /* b200_mla_kv_format, with or without B200_MLA_APPEND_WRITE_STATUS */
+    int32_t reserved;
     void *kv_codes;           /* planes as in b200_mla_decode_args */
     int64_t kv_codes_stride;
     void *kv_block_scales;

@@ -144,3 +144,14 @@ def test_plan_caches_with_threads(monkeypatch):
     [t.join() for t in threads]
     sys.setswitchinterval(old)
     assert not errors
+
+
+def test_append_arguments_of_the_c_entry():
+    """What the reserved word holds does not matter; the flag that asks for the status word is part of kv_format."""
+    from amd_optimization_challenge_b200 import _cabi
+    a = _cabi.KvAppendArgs(rows_bf16=4096, n=3, row_stride=576, num_slots=10, kv_codes=4096, kv_codes_stride=576, base_slot=8, reserved=0x5A5A5A5A)
+    for fmt, error in ((0, b"kv_scale"), (1, b"kv_block_scales"), (2, b"kv_scale"), (3, b"kv_format"), (256, b"status word"), (512, b"kv_format"), (-1, b"kv_format")):
+        a.kv_format = fmt
+        assert _cabi.lib.b200_mla_kv_append(a, None) == -1 and error in _cabi.lib.b200_mla_last_error(), fmt
+    a.kv_format, a.n = 0, 0
+    assert _cabi.lib.b200_mla_kv_append(a, None) == 0
