@@ -433,7 +433,7 @@ int32_t b200_mla_kv_append(const b200_mla_kv_append_args* a, void* stream) {
     if (kv_format == B200_MLA_KV_HYBRID && (!a->kv_rope || ((uintptr_t)a->kv_rope & 15) || a->kv_rope_stride % 16 || a->kv_rope_stride < 64))
         return fail(B200_MLA_ERR_INVALID_ARG, "kv_rope must be 16-byte aligned with a stride >= 64 that is a multiple of 16");
     if (a->num_slots <= 0) return fail(B200_MLA_ERR_INVALID_ARG, "num_slots must be positive");
-    if (!a->slots && (a->base_slot < 0 || a->base_slot + a->n > a->num_slots))
+    if (!a->slots && (a->base_slot < 0 || a->base_slot > a->num_slots - a->n))
         return fail(B200_MLA_ERR_INVALID_ARG, "rows [base_slot, base_slot + n) do not fit in num_slots");
     if (a->slots && !a->status) return fail(B200_MLA_ERR_INVALID_ARG, "status (device int32) is required with a slot list: it reports slots outside the cache");
     cudaError_t e = launch_kv_append(a->rows_bf16, a->n, a->row_stride, a->slots, a->base_slot, a->num_slots, kv_format,

@@ -153,5 +153,9 @@ def test_append_arguments_of_the_c_entry():
     for fmt, error in ((0, b"kv_scale"), (1, b"kv_block_scales"), (2, b"kv_scale"), (3, b"kv_format"), (256, b"status word"), (512, b"kv_format"), (-1, b"kv_format")):
         a.kv_format = fmt
         assert _cabi.lib.b200_mla_kv_append(a, None) == -1 and error in _cabi.lib.b200_mla_last_error(), fmt
+    a.kv_format, a.kv_scale = 0, 4096
+    for base in (-1, 8, 10, (1 << 63) - 1):                      # the last one plus three rows is negative in 64 bits
+        a.base_slot = base
+        assert _cabi.lib.b200_mla_kv_append(a, None) == -1 and b"do not fit" in _cabi.lib.b200_mla_last_error()
     a.kv_format, a.n = 0, 0
     assert _cabi.lib.b200_mla_kv_append(a, None) == 0
