@@ -259,6 +259,10 @@ int32_t b200_mla_decode_static(const b200_mla_decode_args* args, void* stream) {
     void* ptr = nullptr;
     const int rc = static_workspace_ptr(&ptr);
     if (rc != B200_MLA_OK) return rc;
+    // All callers share this scratch.  Calls that overlapped, against the rule, may have left words of the header behind their
+    // status word non-zero, and then every later call would meet too early.
+    const cudaError_t e = cudaMemsetAsync((char*)ptr + 4 * SYNC_AMAX, 0, 256 - 4 * SYNC_AMAX, (cudaStream_t)stream);
+    if (e != cudaSuccess) return fail(B200_MLA_ERR_CUDA, "scratch header reset failed: %s", cudaGetErrorString(e));
     b200_mla_decode_args a = *args;
     a.workspace = ptr;
     a.workspace_bytes = B200_MLA_STATIC_WORKSPACE_BYTES;

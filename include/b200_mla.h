@@ -125,7 +125,8 @@ typedef struct {
     void *workspace;          /* device, 256-byte aligned.  Its first 256 bytes hold the sticky status word and the
                                * words through which the CTAs of a call meet, and must be zero before the first call that
                                * uses a fresh buffer (b200_mla_reset_status, or any memset).  Calls leave all of them but
-                               * the status word at zero */
+                               * the status word at zero.  Calls that share a workspace must not overlap; should they have,
+                               * zero the header again */
     int64_t workspace_bytes;  /* >= b200_mla_workspace_bytes() */
 } b200_mla_decode_args;
 
@@ -233,8 +234,9 @@ int32_t b200_mla_q_amax(const void *x_bf16, int64_t n, uint32_t *parts_out, void
  *     current); make that first call outside any stream capture.
  *   - The call itself performs no cudaMalloc / cudaFree and calls no allocating library routine.
  *   - All calls on a device share the one array: calls that overlap on the GPU (two streams, two
- *     threads) race on the partials.  Contents persist from call to call; nothing in them has to
- *     be cleared by the caller (the status word starts at zero and is sticky).
+ *     threads) race on the partials and on the words through which the CTAs of a call meet, and their results are
+ *     not valid; a call that overlaps with none is not affected by earlier ones that did.  Nothing has to be cleared by the
+ *     caller (the status word starts at zero and is sticky).
  */
 #define B200_MLA_STATIC_WORKSPACE_BYTES (16u << 20)
 int32_t b200_mla_decode_static(const b200_mla_decode_args *args, void *stream);
