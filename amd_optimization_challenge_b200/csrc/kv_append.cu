@@ -132,11 +132,11 @@ __global__ void __launch_bounds__(THREADS, RESIDENT) kv_append_kernel(const Appe
             const int tid = (int)threadIdx.x, head = (int)min((long long)((0u - (unsigned int)(uintptr_t)p.slots) >> 2 & 3u), p.n);
             const long long n4 = (p.n - head) >> 2, tail = head + 4 * n4;
             const int4* s4 = reinterpret_cast<const int4*>(p.slots + head);
-            if (tid < head) any = (unsigned int)__ldg(p.slots + tid) >= top;
-            if (tail + tid < p.n) any |= (unsigned int)__ldg(p.slots + tail + tid) >= top;
+            if (tid < head) any = (unsigned int)__ldcg(p.slots + tid) >= top;
+            if (tail + tid < p.n) any |= (unsigned int)__ldcg(p.slots + tail + tid) >= top;
 #pragma unroll 8
             for (long long i = tid; i < n4; i += THREADS) {
-                const int4 s = __ldg(s4 + i);
+                const int4 s = __ldcg(s4 + i);
                 any |= max(max((unsigned int)s.x, (unsigned int)s.y), max((unsigned int)s.z, (unsigned int)s.w)) >= top;
             }
         }
@@ -158,14 +158,14 @@ __global__ void __launch_bounds__(THREADS, RESIDENT) kv_append_kernel(const Appe
 #pragma unroll
         for (int k = 0; k < VEC; ++k) v[k] = make_uint4(0u, 0u, 0u, 0u);
         if (sub < left) {
-            if (LISTED) slot = (unsigned int)__ldg(list);
+            if (LISTED) slot = (unsigned int)__ldcg(list);
 #pragma unroll
-            for (int k = 0; k < VEC; ++k) v[k] = __ldg(src + k);
+            for (int k = 0; k < VEC; ++k) v[k] = __ldcg(src + k);
         }
         src += src_hop;
         list += hop;
     };
-    const float scale = KVFMT != KV_MXFP4 ? __ldg(p.scale) : 1.0f;
+    const float scale = KVFMT != KV_MXFP4 ? __ldcg(p.scale) : 1.0f;
     fetch();
     const float rscale = __frcp_rn(scale);
     const unsigned int general = general_from(rscale);

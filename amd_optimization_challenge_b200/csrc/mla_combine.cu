@@ -40,17 +40,17 @@ __global__ void __launch_bounds__(128) combine_parts_kernel(const float* __restr
     auto load = [&](int i0) {
 #pragma unroll
         for (int k = 0; k < GROUP; ++k)
-            if (i0 + k < parts) lse[k] = __ldg(lse_parts + (i0 + k) * lse_stride + r);
+            if (i0 + k < parts) lse[k] = __ldcg(lse_parts + (i0 + k) * lse_stride + r);
 #pragma unroll
         for (int k = 0; k < GROUP; ++k)
-            if (i0 + k < parts) v[k] = __ldg(reinterpret_cast<const float4*>(o_parts + (i0 + k) * o_stride + r * V_DIM + d));
+            if (i0 + k < parts) v[k] = __ldcg(reinterpret_cast<const float4*>(o_parts + (i0 + k) * o_stride + r * V_DIM + d));
     };
     load(0);
     float M = -INFINITY;
 #pragma unroll
     for (int k = 0; k < GROUP; ++k)
         if (k < parts) M = fmaxf(M, lse[k]);
-    for (int i = GROUP; i < parts; ++i) M = fmaxf(M, __ldg(lse_parts + i * lse_stride + r));
+    for (int i = GROUP; i < parts; ++i) M = fmaxf(M, __ldcg(lse_parts + i * lse_stride + r));
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     float den = 0.f;
     if (M > -INFINITY) {

@@ -27,7 +27,8 @@ enum { ST_OK = 0, ST_TIMEOUT = 1, ST_BAD_PAGE = 2 };
 
 // Launch of a kernel whose first statement is pdl_wait(): its blocks are placed while the kernel before it in the stream
 // drains, which leaves 1 us between the two instead of 3 us.  pdl_wait returns when that kernel is complete and its writes
-// are visible, so nothing may be read or written before it.  (Cooperative launches do not take the attribute.)
+// are visible, so nothing may be read or written before it.  What that kernel may have written is read with __ldcg: __ldg is for
+// data that nobody writes while the kernel runs, and its blocks run already.  (Cooperative launches do not take the attribute.)
 template <typename... Params, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, unsigned int threads, cudaStream_t stream, Args... args) {
     cudaLaunchAttribute attr;
