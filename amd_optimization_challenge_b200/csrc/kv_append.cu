@@ -64,12 +64,6 @@ __device__ __forceinline__ uint2 cast_e4m3x8(const uint4& v, float scale, float 
     if (max(m & 0xffffu, m >> 16) >= general) return q_cast_e4m3x8(v, scale);
     return make_uint2(c[0] | (c[1] << 16), c[2] | (c[3] << 16));
 }
-// Magnitude bits (exponent field f) below which |x r| < 2^127 and finite: |x| < 2^(f - 126), |r| < 2^(e - 126), e its exponent field.
-__device__ __forceinline__ unsigned int general_from(float r) {
-    const int e = (int)((__float_as_uint(r) >> 23) & 0xffu);
-    return e == 255 ? 0u : (unsigned int)min(380 - e, 255) << 7;
-}
-
 // Eight bf16 values of a 32-element block whose other values are in the lanes of the same aligned group of four -> eight
 // e2m1 codes and the block's E8M0 byte.  All 32 lanes call it.
 __device__ __forceinline__ uint32_t quant_mxfp4x8(const uint4& v, uint8_t& scale_byte) {

@@ -301,6 +301,12 @@ __device__ __forceinline__ uint8_t q_cast_e4m3(__nv_bfloat16 x, float scale) {
     const float y = fminf(fmaxf(q_quotient_bf16(__bfloat162float(x), scale, __frcp_rn(scale)), -448.0f), 448.0f);
     return (uint8_t)__nv_cvt_float_to_fp8(y, __NV_SATFINITE, __NV_E4M3);
 }
+// Magnitude bits (exponent field f) of a bf16 x below which |x r| < 2^127 and finite: |x| < 2^(f - 126), |r| < 2^(e - 126), e the
+// exponent field of r = RN(1 / scale).  Such quotients need no special cases.
+__device__ __forceinline__ unsigned int general_from(float r) {
+    const int e = (int)((__float_as_uint(r) >> 23) & 0xffu);
+    return e == 255 ? 0u : (unsigned int)min(380 - e, 255) << 7;
+}
 // eight bf16 values (one 16-byte vector) -> eight e4m3 bytes
 __device__ __forceinline__ uint2 q_cast_e4m3x8(const uint4& v, float scale) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};             // by value: the vector stays in registers

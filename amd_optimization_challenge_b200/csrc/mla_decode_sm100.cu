@@ -296,8 +296,8 @@ __device__ __forceinline__ unsigned int bf16x8_amax_bits(const uint4& v) {
 }
 __device__ __forceinline__ f32x2 bf16x2_to_f32x2(uint32_t w) { return pk2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 // eight bf16 values -> the eight e4m3 codes of q_cast_e4m3x8 (mla_common.cuh) in half the instructions: s2 = -scale and
-// r2 = RN(1 / scale), twice.  No value of a tensor exceeds its own scale's range, so the quotient needs no special cases,
-// and a -0 may come out as +0 (no product or sum of the decode tells them apart).
+// r2 = RN(1 / scale), twice.  For values below general_from(r), which those of a tensor are of its own scale; a -0 may come out
+// as +0 (no product or sum of the decode tells them apart).
 __device__ __forceinline__ uint2 q_quant_e4m3x8(const uint4& v, f32x2 s2, f32x2 r2) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     uint32_t q[4];
@@ -507,8 +507,20 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                             // an infinite scale (infinite Q) gives zeros and NaNs as the division would
                             const float rs = __frcp_rn(q_scale), sn = q_scale <= 3.0e38f ? -q_scale : 0.0f;
                             const f32x2 r2 = pk2(rs, rs), s2 = pk2(sn, sn);
+                            bool special = false;
+                            if (!own_amax) {                      // the caller's maxima: there may be values far beyond them
+                                unsigned int m = 0;
 #pragma unroll
-                            for (int u = 0; u < 9; ++u) *dst(u) = q_quant_e4m3x8(raw[u], s2, r2);
+                                for (int u = 0; u < 9; ++u) m = max(m, bf16x8_amax_bits(raw[u]));
+                                special = m >= general_from(rs);
+                            }
+                            if (special) {
+#pragma unroll 1
+                                for (int u = 0; u < 9; ++u) *dst(u) = q_cast_e4m3x8(__ldg(src + 8 * u), q_scale);
+                            } else {
+#pragma unroll
+                                for (int u = 0; u < 9; ++u) *dst(u) = q_quant_e4m3x8(raw[u], s2, r2);
+                            }
                         }
                     }
                 } else {

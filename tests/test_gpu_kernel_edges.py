@@ -458,3 +458,18 @@ def test_append_reports_a_bad_slot_wherever_it_stands(pkg, n, off):
             assert int(pkg.kv_append(rows, "mxfp4", planes, slots=slots)) == 1
         slots[i] = i
     assert int(pkg.kv_append(rows, "mxfp4", planes, slots=slots)) == 0
+
+
+@pytest.mark.parametrize("heads", [16, 32, 64])
+@pytest.mark.parametrize("impl", ["tcgen05", "generic"])
+def test_q_cast_with_values_beyond_the_given_maxima(pkg, impl, heads):
+    """The caller's maxima may be those of another tensor: what lies beyond saturates, infinities included."""
+    data = pkg.generate_input(3, 1, 200, seed=12, num_heads=heads, formats=("fp8",))
+    q, kvd, _, ip, cfg = data
+    parts, top = pkg.q_amax_parts(q).clone(), float(q.float().abs().max())
+    wild, tame = q.clone(), q.clone()
+    for (b, h, d), x in (((0, 3, 10), float("inf")), ((0, 9, 571), -3.0e38), ((1, 15, 511), float("-inf")), ((2, 0, 0), 1.0e30), ((2, 5, 64), 50 * top)):
+        wild[b, h, d], tame[b, h, d] = x, top if x > 0 else -top
+    run = lambda t: pkg.mla_decode(t, parts, "fp8", kvd["fp8"], ip, sm_scale=0.01, q_cast=True, impl=impl)
+    assert torch.isfinite(run(wild).float()).all()
+    assert torch.equal(run(wild), run(tame))
