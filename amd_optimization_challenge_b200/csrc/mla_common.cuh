@@ -237,7 +237,8 @@ __device__ __forceinline__ int page_of(const MlaParams& p, int pos) { return p.p
 __device__ __forceinline__ int off_in_page(const MlaParams& p, int pos) { return p.page_shift >= 0 ? pos & (p.page_size - 1) : pos % p.page_size; }
 // Row of the cache planes that is actually read for slot `s`: s itself inside [0, num_slots), else a row inside
 // (negative values, the "no row" marker -1 included, map to the last row).  Nothing outside the planes is ever read;
-// a key whose id needed the clamp reads as some other row, which check_span_pages reports as ST_BAD_PAGE.  The
+// a key whose id needed the clamp reads as some other row, which is reported as ST_BAD_PAGE (by the tcgen05 kernels where the id
+// becomes an address, by the warp-level kernel in check_span_pages).  The
 // clamp is applied where a slot is turned into an address, not where it is loaded: the kernels load page ids one or
 // two steps ahead of their use, and touching the value early would wait for that load (measured: 10-25 % of a call).
 __device__ __forceinline__ unsigned int clamp_slot(const MlaParams& p, int s) { return min((unsigned int)s, p.last_slot); }
@@ -296,10 +297,6 @@ __device__ __forceinline__ float q_quotient_bf16(float x, float scale, float rsc
     if (!(fabsf(t) <= 3.0e38f)) y = t;                                        // infinite / NaN input
     y = copysignf(fabsf(y), x);
     return __bfloat162float(__float2bfloat16_rn(y));
-}
-__device__ __forceinline__ uint8_t q_cast_e4m3(__nv_bfloat16 x, float scale) {
-    const float y = fminf(fmaxf(q_quotient_bf16(__bfloat162float(x), scale, __frcp_rn(scale)), -448.0f), 448.0f);
-    return (uint8_t)__nv_cvt_float_to_fp8(y, __NV_SATFINITE, __NV_E4M3);
 }
 // Magnitude bits (exponent field f) of a bf16 x below which |x r| < 2^127 and finite: |x| < 2^(f - 126), |r| < 2^(e - 126), e the
 // exponent field of r = RN(1 / scale).  Such quotients need no special cases.

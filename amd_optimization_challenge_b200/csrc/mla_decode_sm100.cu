@@ -344,7 +344,7 @@ __device__ __forceinline__ uint32_t operand_offset(int r, int c) {
 
 template <int N, int KVFMT, int QFMT>
 __global__ void __launch_bounds__(Cfg<N, KVFMT, QFMT>::THREADS, 1)
-mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, const int use_tma) {
+mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, const bool use_tma) {
     using C = Cfg<N, KVFMT, QFMT>;
     constexpr int NQ = C::NQ, NC = C::NC, SW = C::SW, FW = C::FW, TILE = C::TILE, NS = C::NS, UNITS = C::UNITS;
     constexpr int PANEL_BYTES = C::PANEL_BYTES, STAGE_BYTES = C::STAGE_BYTES, P_BUFS = C::P_BUFS;
@@ -1192,7 +1192,6 @@ cudaError_t launch_cfg(const MlaParams& p, cudaStream_t stream) {
     const sm100::Maps* maps = nullptr;
     const char* off = getenv("B200_MLA_DISABLE_TMA");                 // testing aid: "1" keeps every tile on the copy loop
     if (KVFMT == KV_E4M3 && !(off && off[0] == '1')) maps = cache_maps(p);
-    const int use_tma = !maps ? 0 : (p.kv_indices == nullptr ? 1 : 2);
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeCooperative;
     attr.val.cooperative = 1;
@@ -1203,7 +1202,7 @@ cudaError_t launch_cfg(const MlaParams& p, cudaStream_t stream) {
     cfg.stream = stream;
     cfg.attrs = &attr;
     cfg.numAttrs = p.fused ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, p, maps ? *maps : no_maps, use_tma);
+    return cudaLaunchKernelEx(&cfg, kernel, p, maps ? *maps : no_maps, maps != nullptr);
 }
 
 template <int KVFMT>

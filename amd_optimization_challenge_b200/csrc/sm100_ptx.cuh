@@ -32,15 +32,6 @@ __device__ __forceinline__ bool mbar_try_for(uint64_t* bar, uint32_t parity, uin
     return ok != 0;
 }
 __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) { return mbar_try_for(bar, parity, 20000u); }
-__device__ __forceinline__ bool mbar_try_nb(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
 // Wait for completion number `n` (0-based) of the barrier; n = -1 passes at once.
 // The wait is bounded: when it expires the thread raises the CTA's abort flag and carries on, and
 // every later wait of the CTA returns at once.  Control flow never depends on the outcome, so all
@@ -142,16 +133,6 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t cols) {
 __device__ __forceinline__ void tmem_relinquish() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 // Warp-wide forms: every lane of a converged warp executes them and one elected lane (the same one every time for a
 // full mask) issues the instruction.  The surrounding loop then runs warp-uniformly, which keeps the descriptor
