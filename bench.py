@@ -10,8 +10,8 @@ KV length 4096, page size 1 behind a shuffled page table).
 
 Prints ONE JSON line (rank 0).  Keys beyond the base contract:
   us_per_call, achieved_gbs   the other two forms of the headline metric
-  roofline                    the stage-1 kernel: algorithmic bytes per launch / its CUDA-event
-                              duration, against the measured HBM copy bandwidth
+  roofline                    the decode launch (maximum of Q, split-KV decode, merge): algorithmic bytes per
+                              launch / its CUDA-event duration, against the measured HBM copy bandwidth
   cpu_baseline                the CPU oracle (torch fp32 dequantise-then-attend) timed on this host
   e2e                         the same call with every input staged from pinned host memory and
                               the output copied back, copies inside the timed region
@@ -53,7 +53,7 @@ KV_ROW_BYTES = {"fp8": 576, "mxfp4": 306, "hybrid": 336}
 # how a workload uses N > 1 GPUs: independent replicas (weak scaling), a token-balanced split of the
 # batch (strong, no collective), or each sequence's keys split over the GPUs (strong, one all-gather)
 MODES = {"c1": "replica", "c2": "replica", "c3": "batch_shard", "c4": "split_kv"}
-# DRAM bytes read + written by one stage-1 launch, from one ncu capture of that workload's kernel on one GPU
+# DRAM bytes read + written by one decode launch, from one ncu capture of that workload's kernel on one GPU
 # (profiles/ holds each capture's summary and command; regenerate them together with the kernels).
 NCU_TRAFFIC_BYTES = {"c1": 77.8e6, "c2": 190.0e6, "c3": 606.5e6, "c4": 427.9e6}
 L2_BYTES = 126 << 20
@@ -189,7 +189,7 @@ def _gpu_time_us(fn, steps, dev, dist=None, world=1, spin_cycles=int(4e7)):
 
 
 def _stage1_us(pkg, fn, reps, dev, dist=None, world=1):
-    """Mean duration of the stage-1 launch inside `fn` (events recorded by the library), max over ranks."""
+    """Mean duration of the decode launch inside `fn` (events recorded by the library), max over ranks."""
     lib = pkg._cabi.lib
     pairs = []
     for _ in range(reps):
@@ -236,7 +236,7 @@ def sharded_modes(pkg, dist, rank, world, dev, kernel="auto", steps=30):
     out["c3"] = {"mode": "token-balanced batch shard, no collective", "us_per_step": tn, "tokens_per_s": tokens / (tn * 1e-6),
                  "stage1_us_max_rank": s1, "n1_us_per_step": t1, "speedup_vs_n1": t1 / tn,
                  "efficiency_vs_n1": t1 / tn / world, "kv_tokens_per_rank": {"min": min(loads), "max": max(loads)},
-                 "limiter": "stage-1 kernel of the most loaded rank (no exchange step)"}
+                 "limiter": "decode launch of the most loaded rank (no exchange step)"}
     del full, mine
     torch.cuda.empty_cache()
 
@@ -487,7 +487,7 @@ def main():
 
     host = build_host(1234 + rank, rank, world, mode)
     w_rank = dict(w, batch=host["batch"])
-    abytes = algorithmic_bytes(w_rank, host["total_kv"])       # this rank's stage-1 launch
+    abytes = algorithmic_bytes(w_rank, host["total_kv"])       # this rank's decode launch
     tokens_job = tokens_per_call if mode != "replica" else n_gpus * tokens_per_call
     kv_bytes = sum(t.numel() * t.element_size() for t in host["kv"])
     n_rot = max(2, -(-int(2.4 * L2_BYTES) // kv_bytes))         # rotate > 2.4x L2 worth of cache copies
@@ -594,7 +594,7 @@ def main():
     ms_per_step = ms / args.steps
     value = tokens_job / (ms_per_step * 1e-3)
 
-    # ---- stage-1 kernel duration (CUDA events recorded by the library around that launch)
+    # ---- duration of the decode launch (CUDA events recorded by the library around that launch)
     lib = pkg._cabi.lib
     k_ms = []
     pairs = []
@@ -617,7 +617,7 @@ def main():
     hbm = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
            "traffic": NCU_TRAFFIC_BYTES.get(args.workload) if mode == "replica" else None,
            "traffic_unit": "bytes per launch (ncu dram read + write, separate capture of this kernel; profiles/)",
-           "kernel": "mla_decode stage 1", "kernel_us": k_us,
+           "kernel": "mla_decode (maximum of Q, split-KV decode and merge in one launch)", "kernel_us": k_us,
            "algorithmic_bytes": abytes, "peak_source": f"of {peak_kind}"}
     if w["heads"] >= 128:
         # the H = 128 shape is bound by the tensor pipe, not by HBM: report it against the dense e4m3 rate

@@ -273,7 +273,8 @@ int32_t b200_mla_graph_status(int32_t word, int32_t *out, void *stream);
 /*
  * Profiling aid (no counterpart in the reference, whose harness times whole calls, eval.py:225-261):
  * while both events (cudaEvent_t) are non-NULL, every b200_mla_decode issued by the calling thread
- * records `start` before and `stop` after its stage-1 kernel on the call's stream.  Pass NULLs to
+ * records `start` before and `stop` after its decode launch on the call's stream (with the maximum of Q and the merge where
+ * they are part of that launch).  Pass NULLs to
  * switch it off.
  */
 int32_t b200_mla_set_stage1_events(void *start_event, void *stop_event);
