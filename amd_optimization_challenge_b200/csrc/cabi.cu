@@ -2,6 +2,7 @@
 // and launches.  Declarations and the reference interfaces they replace: include/b200_mla.h.
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 
 #include "../../include/b200_mla.h"
@@ -61,15 +62,11 @@ int sm_count() {
     return cached;
 }
 
-bool cooperative_ok() {
-    static thread_local int cached_dev = -1, cached = 0;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return false;
-    if (dev != cached_dev) {
-        if (cudaDeviceGetAttribute(&cached, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess) cached = 0;
-        cached_dev = dev;
-    }
-    return cached != 0;
+// MlaParams::meet_cycles: 50 us at 2 GHz, well above what the CTAs of a call are apart (they get equal shares; measured:
+// up to 10 us).  Testing aid: B200_MLA_MEET_CYCLES, 0 makes every CTA leave at once.
+int meet_cycles() {
+    const char* e = getenv("B200_MLA_MEET_CYCLES");
+    return e && e[0] ? atoi(e) : 100000;
 }
 
 constexpr int kMaxCtasPerSm = 2;
@@ -191,9 +188,10 @@ int32_t b200_mla_decode(const b200_mla_decode_args* a, void* stream_) {
     p.part_lse = (float*)(ws + L.lse_off);
     p.part_o = (float*)(ws + L.o_off);
 
-    // One cooperative launch for everything - the maximum of Q, the decode, the merge - where all its CTAs are resident at
-    // once (one per SM); else the pieces as kernels of their own.
-    p.fused = use_sm100 && (long long)G * groups <= sms && cooperative_ok();
+    // One launch for everything - the maximum of Q, the decode, the merge - where the GPU holds all its CTAs at once (one per
+    // SM); else the pieces as kernels of their own.
+    p.fused = use_sm100 && (long long)G * groups <= (sms < MAX_FUSED_CTAS ? sms : MAX_FUSED_CTAS);
+    p.meet_cycles = meet_cycles();
     cudaError_t e = cudaSuccess;
     if (quant && !p.fused) {
         unsigned int* parts = (unsigned int*)(ws + L.amax_off);

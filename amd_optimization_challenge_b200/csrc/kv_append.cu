@@ -198,7 +198,7 @@ template <int KVFMT>
 cudaError_t launch_format(const AppendParams& p, cudaStream_t stream) {
     const long long wave = 148 * RESIDENT, steps = (p.n + block_rows(KVFMT) - 1) / block_rows(KVFMT), cap = steps <= 8 * wave ? wave : 4 * wave;
     const unsigned int blocks = (unsigned int)(steps < cap ? steps : cap) + (unsigned int)p.write_status;
-    return launch_pdl(p.slots ? kv_append_kernel<KVFMT, true> : kv_append_kernel<KVFMT, false>, blocks, THREADS, stream, p);
+    return launch_pdl(p.slots ? kv_append_kernel<KVFMT, true> : kv_append_kernel<KVFMT, false>, blocks, THREADS, 0, stream, p);
 }
 
 }  // namespace

@@ -75,13 +75,13 @@ __global__ void __launch_bounds__(128) combine_parts_kernel(const float* __restr
 
 cudaError_t launch_combine_spans(const MlaParams& p, cudaStream_t stream) {
     dim3 grid(p.batch, p.rows);
-    return launch_pdl(combine_spans_kernel, grid, 128, stream, p);
+    return launch_pdl(combine_spans_kernel, grid, 128, 0, stream, p);
 }
 
 cudaError_t launch_combine_parts(const float* o_parts, const float* lse_parts, int parts, long long rows,
                                  long long o_stride, long long lse_stride, __nv_bfloat16* out, float* out_lse,
                                  cudaStream_t stream) {
-    return launch_pdl(combine_parts_kernel, dim3((unsigned)rows), 128, stream, o_parts, lse_parts, parts, rows, o_stride, lse_stride, out,
+    return launch_pdl(combine_parts_kernel, dim3((unsigned)rows), 128, 0, stream, o_parts, lse_parts, parts, rows, o_stride, lse_stride, out,
                       out_lse);
 }
 

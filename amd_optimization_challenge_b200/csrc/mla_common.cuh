@@ -27,23 +27,26 @@ enum { ST_OK = 0, ST_TIMEOUT = 1, ST_BAD_PAGE = 2 };
 
 // Launch of a kernel whose first statement is pdl_wait(): its blocks are placed while the kernel before it in the stream
 // drains, which leaves 1 us between the two instead of 3 us.  pdl_wait returns when that kernel is complete and its writes
-// are visible, so nothing may be read or written before it.  What that kernel may have written is read with __ldcg: __ldg is for
-// data that nobody writes while the kernel runs, and its blocks run already.  (Cooperative launches do not take the attribute.)
+// are visible, so nothing may be read or written before it.  What that kernel may have written is read with __ldcg or
+// load_global: __ldg is for data that nobody writes while the kernel runs, and its blocks run already.
 template <typename... Params, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, unsigned int threads, cudaStream_t stream, Args... args) {
+inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, unsigned int threads, unsigned int smem, cudaStream_t stream, const Args&... args) {
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.stream = stream; cfg.attrs = &attr; cfg.numAttrs = 1;
+    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream; cfg.attrs = &attr; cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
+template <typename T>
+__device__ __forceinline__ T load_global(const T* p) { return *p; }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Words of the 256-byte workspace header behind the status word.  ST_FORWARD: address (two words) of a second status word that
 // receives the same bits, 0 if there is none.  SYNC_*: for launches whose CTAs work together; they are zero between launches:
-// the last CTA to leave resets them.
-enum { ST_FORWARD = 2, SYNC_AMAX = 16, SYNC_AMAX_COUNT = 17, SYNC_PREFIX = 18, SYNC_ARRIVE = 32, SYNC_EXIT = 48 };
+// the last CTA to exit resets them.  SYNC_LEFT: one bit per CTA.
+enum { ST_FORWARD = 2, SYNC_AMAX = 16, SYNC_AMAX_COUNT = 17, SYNC_PREFIX = 18, SYNC_ARRIVE = 32, SYNC_EXIT = 48, SYNC_LEFT = 52, SYNC_LEFT_WORDS = 8 };
+constexpr int MAX_FUSED_CTAS = 32 * SYNC_LEFT_WORDS;
 
 struct MlaParams {
     int batch, heads, q_len, rows;      // rows = q_len * heads (query rows per sequence)
@@ -74,7 +77,13 @@ struct MlaParams {
     int q_cast;                         // q is bf16 and is quantised to e4m3 (per-tensor, reference rule) as it is loaded;
     const unsigned int* q_amax_parts;   //   its scale comes from these Q_AMAX_PARTS partial maxima (bf16 bit patterns),
                                         //   or, nullptr, from the maximum the CTAs of the launch find together (SYNC_AMAX)
-    int fused;                          // the launch is cooperative: its CTAs also merge the partials, after a grid-wide barrier
+    int fused;                          // the CTAs of the launch also merge the partials, where they meet
+    // How long a CTA waits for the others of its launch, twice: for the maximum of Q and before the merge.  They are all resident at
+    // once unless something else holds SMs, but nothing depends on it: when the time is up, the CTA looks at all of Q itself, and
+    // leaves its share of the merge to the last CTA to arrive.  So the launch need not be cooperative, and it can overlap with the
+    // end of the kernel before it (launch_pdl): 0.8 us between two kernels instead of 2.1, and no rounding up to ticks of 1 or 2 us,
+    // which is how other launches of a stream start (e4m3 4 x 1024 12.3 -> 10.0 us a call, 32 x 4096 26.3 -> 23.9).
+    int meet_cycles;
 };
 
 // ---------------------------------------------------------------------------------------------

@@ -51,12 +51,15 @@ constexpr int RAW_MAX = 10;               // landing buffers of a block-scaled c
 constexpr int SMEM_LIMIT = 232448;        // opt-in shared memory per CTA
 constexpr int E_BIAS = 127 + 6;           // operand bytes of a block-scaled unit are in units of 2^(E_unit - E_BIAS)
 
+enum { MEET_LEAVE = 0, MEET_ALL = 1, MEET_OTHERS = 2 };
+
 struct Misc {
     uint64_t kv_full[NS_MAX], kv_empty[NS_MAX][4], s_full[2], s_empty[2], p_full[2], p_empty[2], q_full, o_free;
     uint64_t raw_full[RAW_MAX], raw_empty[RAW_MAX];
     int raw_slot[RAW_MAX][UNIT_TOK];      // cache rows of the unit in each landing buffer
     uint32_t tmem_base;
     int abort_flag;
+    int meet, left[SYNC_LEFT_WORDS];      // outcome of the CTAs' meeting (MEET_*), the CTAs that have left before it
     int span[4];                          // first sequence, its first global tile, first and end tile of this CTA
     unsigned int q_red[8];                // cross-warp maximum of a split Q
     long long q_off[4];                   // element offset of each 16-row chunk of this row group inside a sequence's Q
@@ -186,7 +189,7 @@ __device__ __forceinline__ int tiles_of_len(int len) { return len > 0 ? (len + T
 
 template <int TILE>
 __device__ __forceinline__ int seq_tiles(const int* ip, int b, int end) {
-    return b < end ? tiles_of_len<TILE>(__ldg(ip + b + 1) - __ldg(ip + b)) : 0;
+    return b < end ? tiles_of_len<TILE>(load_global(ip + b + 1) - load_global(ip + b)) : 0;
 }
 __device__ __forceinline__ int warp_scan(int v, int lane) {
 #pragma unroll
@@ -255,8 +258,8 @@ struct Walk {
         if (t < t1) return false;
         do {
             ++b;
-            base = __ldg(p.kv_indptr + b);
-            len = max(__ldg(p.kv_indptr + b + 1) - base, 0);
+            base = load_global(p.kv_indptr + b);
+            len = max(load_global(p.kv_indptr + b + 1) - base, 0);
             t0 = t1;
             t1 = t0 + tiles_of_len<TILE>(len);
         } while (t1 <= t);
@@ -359,15 +362,8 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
     // Q quantised by this launch: its CTAs find the largest magnitude together, each in its share of Q
     const bool own_amax = !C::QSPLIT && p.q_cast && p.q_amax_parts == nullptr;
 
-    if (warp == C::AUX_WARP) {
-        int span[4];
-        find_span<TILE>(p, w, G, lane, span, w == 0 && blockIdx.y == 0);
-        if (lane < 4) ms.span[lane] = lane == 0 ? span[0] : (lane == 1 ? span[1] : (lane == 2 ? span[2] : span[3]));
-        if (lane < N / 16) {
-            const int r = row0 + 16 * lane, j = r / p.heads;
-            ms.q_off[lane] = (long long)j * p.q_row_stride + (long long)(r - j * p.heads) * p.q_head_stride;
-        }
-    } else if (warp == C::QK_WARP) {
+    // Nothing of this touches memory that the kernel before may still write: it runs while that one drains.
+    if (warp == C::QK_WARP) {
         tmem_alloc(&ms.tmem_base, C::TMEM_COLS);
         tmem_relinquish();
     } else if (tid == 32 * SW) {
@@ -388,6 +384,17 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
     } else if (tid == 32 * (SW + 1) && use_tma) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.lat) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.rope) : "memory");
+    }
+    __syncwarp();
+    pdl_wait();
+    if (warp == C::AUX_WARP) {
+        int span[4];
+        find_span<TILE>(p, w, G, lane, span, w == 0 && blockIdx.y == 0);
+        if (lane < 4) ms.span[lane] = lane == 0 ? span[0] : (lane == 1 ? span[1] : (lane == 2 ? span[2] : span[3]));
+        if (lane < N / 16) {
+            const int r = row0 + 16 * lane, j = r / p.heads;
+            ms.q_off[lane] = (long long)j * p.q_row_stride + (long long)(r - j * p.heads) * p.q_head_stride;
+        }
     } else if (warp > SW + 1 && warp <= SW + 3 && paged && p.total_kv_hint > 0 && p.total_kv_hint < (1LL << 31)) {
         // The page ids this CTA will walk lie near w/G of the table: pull that neighbourhood into L2 while the span is
         // being searched, so that the first dependent page-table read is not a cold DRAM access.
@@ -404,7 +411,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
         for (unsigned long long i = n8 * c / n_cta + tid; i < end; i += BATCH * ST) {
             uint4 v[BATCH];
 #pragma unroll
-            for (int k = 0; k < BATCH; ++k) v[k] = i + k * ST < end ? __ldg(q8 + i + k * ST) : make_uint4(0u, 0u, 0u, 0u);
+            for (int k = 0; k < BATCH; ++k) v[k] = i + k * ST < end ? __ldcg(q8 + i + k * ST) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
             for (int k = 0; k < BATCH; ++k) m = max(m, bf16x8_amax_bits(v[k]));
         }
@@ -435,17 +442,17 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
             const int sg = C::SMG == 1 ? 0 : warp >> 2, wv = warp & 3, tok = tid & 127, col0 = sg * NC, bar_id = 1 + sg;
             const bool active = wv < TILE / 32;
             const uint32_t lane_base = (uint32_t)(wv * 32) << 16;
-            const float kv_tensor_scale = KVFMT != KV_MXFP4 ? __ldg(p.kv_scale) : 1.0f;
+            const float kv_tensor_scale = KVFMT != KV_MXFP4 ? __ldcg(p.kv_scale) : 1.0f;
             float q_scale = 1.0f;
             bool q_scale_due = own_amax;
             if constexpr (!C::QSPLIT) {
                 if (p.q_cast && !own_amax) {                      // every warp reduces the partial maxima itself
                     unsigned int m = 0;
 #pragma unroll
-                    for (int i = 0; i < Q_AMAX_PARTS / 32; ++i) m = max(m, __ldg(p.q_amax_parts + lane + 32 * i));
+                    for (int i = 0; i < Q_AMAX_PARTS / 32; ++i) m = max(m, __ldcg(p.q_amax_parts + lane + 32 * i));
                     q_scale = q_scale_from_amax_bits(__reduce_max_sync(0xffffffffu, m));
                 } else if (!p.q_cast) {
-                    q_scale = __ldg(p.q_scale);
+                    q_scale = __ldcg(p.q_scale);
                 }
             }
 
@@ -467,7 +474,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                         const uint4* src = reinterpret_cast<const uint4*>(q0 + ms.q_off[r >> 4] + (long long)(r & 15) * p.q_head_stride) + cl;
                         uint4 raw[9];
 #pragma unroll
-                        for (int u = 0; u < 9; ++u) raw[u] = __ldg(src + 8 * u);
+                        for (int u = 0; u < 9; ++u) raw[u] = __ldcg(src + 8 * u);
                         unsigned char* even = q_smem + r * 128 + (((cl >> 1) ^ (r & 7)) << 4) + (cl & 1) * 8;
                         unsigned char* odd = q_smem + r * 128 + (((cl >> 1) ^ 4 ^ (r & 7)) << 4) + (cl & 1) * 8;
                         unsigned char* rope = q_smem + 4 * C::Q_PANEL_BYTES + r * 64 + (((cl >> 1) ^ ((r >> 1) & 3)) << 4) + (cl & 1) * 8;
@@ -496,12 +503,26 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                             }
                         } else {
                             if (q_scale_due) {                    // first use of the scale all CTAs contribute to: by now it is there
-                                if (tid == 0) {
-                                    grid_wait(p.status + SYNC_AMAX_COUNT, (int)(gridDim.x * gridDim.y), abort_flag);
-                                    ms.q_red[0] = *reinterpret_cast<volatile unsigned int*>(p.status + SYNC_AMAX);
-                                }
+                                if (tid == 0)
+                                    ms.q_red[0] = count_reached(p.status + SYNC_AMAX_COUNT, (int)(gridDim.x * gridDim.y), p.meet_cycles)
+                                                      ? *reinterpret_cast<volatile unsigned int*>(p.status + SYNC_AMAX) : 0xffffffffu;
                                 named_bar_sync(3, ST);
-                                q_scale = q_scale_from_amax_bits(ms.q_red[0]);
+                                unsigned int m = ms.q_red[0];
+                                if (m == 0xffffffffu) {           // not all CTAs run yet: this one looks at all of Q itself
+                                    const uint4* q8 = reinterpret_cast<const uint4*>(p.q);
+                                    m = 0;
+#pragma unroll 2
+                                    for (unsigned long long i = tid; i < (unsigned long long)p.batch * p.rows * 72; i += ST) m = max(m, bf16x8_amax_bits(__ldcg(q8 + i)));
+                                    m = __reduce_max_sync(0xffffffffu, m);
+                                    named_bar_sync(3, ST);        // q_red[0] has been read
+                                    if (lane == 0) ms.q_red[warp] = m;
+                                    named_bar_sync(3, ST);
+#pragma unroll
+                                    for (int k = 0; k < SW; ++k) m = max(m, ms.q_red[k]);
+#pragma unroll
+                                    for (int u = 0; u < 9; ++u) raw[u] = __ldcg(src + 8 * u);     // again: not kept over the loop
+                                }
+                                q_scale = q_scale_from_amax_bits(m);
                                 q_scale_due = false;
                             }
                             // an infinite scale (infinite Q) gives zeros and NaNs as the division would
@@ -516,7 +537,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                             }
                             if (special) {
 #pragma unroll 1
-                                for (int u = 0; u < 9; ++u) *dst(u) = q_cast_e4m3x8(__ldg(src + 8 * u), q_scale);
+                                for (int u = 0; u < 9; ++u) *dst(u) = q_cast_e4m3x8(__ldcg(src + 8 * u), q_scale);
                             } else {
 #pragma unroll
                                 for (int u = 0; u < 9; ++u) *dst(u) = q_quant_e4m3x8(raw[u], s2, r2);
@@ -531,7 +552,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                         const uint4* src = reinterpret_cast<const uint4*>(q0 + ms.q_off[r >> 4] + (long long)(r & 15) * p.q_head_stride) + cl;
                         uint4 raw[9];
 #pragma unroll
-                        for (int u = 0; u < 9; ++u) raw[u] = __ldg(src + 4 * u);
+                        for (int u = 0; u < 9; ++u) raw[u] = __ldcg(src + 4 * u);
 #pragma unroll
                         for (int u = 0; u < 9; ++u)
                             *reinterpret_cast<uint4*>(q_smem + (u < 8 ? (u >> 1) * C::Q_PANEL_BYTES + r * 128 + ((((u & 1) << 2 | cl) ^ (r & 7)) << 4)
@@ -619,8 +640,8 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
 #pragma unroll
                     for (int c = 0; c < NC / 2; ++c) l_acc[c] = 0ull;
                     lim_min = 0x7fffffff;
-                    const int pos_off = p.kv_pos_offset ? __ldg(p.kv_pos_offset + wk.b) : 0;
-                    const int tot_len = p.kv_total_len ? __ldg(p.kv_total_len + wk.b) : wk.len;
+                    const int pos_off = p.kv_pos_offset ? __ldcg(p.kv_pos_offset + wk.b) : 0;
+                    const int tot_len = p.kv_total_len ? __ldcg(p.kv_total_len + wk.b) : wk.len;
 #pragma unroll
                     for (int q = 0; q < NC / 16; ++q) {
                         const int j = (row0 + col0 + 16 * q) / p.heads;
@@ -827,10 +848,10 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                 const bool boxes = use_tma && (!paged || p.page_size % UNIT_TOK == 0);
                 int g2 = g, k2 = k;                                   // unit whose page ids are fetched next
                 auto fetch_id = [&]() {
-                    if (wk.seek(p, t_begin + g2)) page_base = p.kv_page_indptr ? __ldg(p.kv_page_indptr + wk.b) : wk.base;
+                    if (wk.seek(p, t_begin + g2)) page_base = p.kv_page_indptr ? load_global(p.kv_page_indptr + wk.b) : wk.base;
                     const int pos0 = (t_begin + g2 - wk.t0) * TILE + k2 * UNIT_TOK, pos = min(pos0 + (lane & 15), wk.len - 1);
                     inside = pos0 + UNIT_TOK <= wk.len;
-                    id = paged ? __ldg(p.kv_indices + page_base + page_of(p, pos)) : wk.base + pos;
+                    id = paged ? load_global(p.kv_indices + page_base + page_of(p, pos)) : wk.base + pos;
                     off = paged ? off_in_page(p, pos) : 0;
                     advance(g2, k2);
                 };
@@ -1034,11 +1055,11 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
             // this loop spent 600 of its 1300 cycles there).
             int id[2], off[2];
             auto look_up = [&](int g) {
-                if (wk.seek(p, t_begin + g)) page_base = p.kv_page_indptr ? __ldg(p.kv_page_indptr + wk.b) : wk.base;
+                if (wk.seek(p, t_begin + g)) page_base = p.kv_page_indptr ? load_global(p.kv_page_indptr + wk.b) : wk.base;
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     const int pos = min((t_begin + g - wk.t0) * TILE + ((4 * i + ((lane >> 4) << 1)) + aw) * UNIT_TOK + (lane & 15), wk.len - 1);
-                    id[i] = paged ? __ldg(p.kv_indices + page_base + page_of(p, pos)) : wk.base + pos;
+                    id[i] = paged ? load_global(p.kv_indices + page_base + page_of(p, pos)) : wk.base + pos;
                     off[i] = paged ? off_in_page(p, pos) : 0;
                 }
             };
@@ -1088,42 +1109,79 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
         }
     }
 
+    // Merge of the partials by the same launch: the CTAs meet, then the query rows are dealt out to all warps - whole rows,
+    // halves or quarters, so that every warp has one item at most where there are few.  (A second kernel cost 5 us and more per
+    // call: launch, drain, cold code.)  The first items go to the warps that are done before the epilogue: they look up
+    // what theirs consists of while the softmax warps still write (three dependent loads, 2 k cycles behind the meeting before).
+    // The launch is not cooperative (see MlaParams::meet_cycles): a CTA that has waited meet_cycles for the others leaves its share
+    // to the last one to arrive.  Whoever comes last sees who has left: a bit in SYNC_LEFT, then the count in the upper half of
+    // SYNC_ARRIVE.  A CTA that learns from that count that all have come after all merges its share too; its bit may have been
+    // seen, and then both write the same values.
+    constexpr int WARPS = C::THREADS / 32;
+    const int n_cta = (int)(gridDim.x * gridDim.y), cta = (int)(blockIdx.y * gridDim.x + blockIdx.x);
+    const int rows_all = p.batch * p.rows, n_warps = n_cta * WARPS;
+    const int sh = rows_all * 4 <= n_warps ? 2 : (rows_all * 2 <= n_warps ? 1 : 0);
+    const int first_item = (warp >= SW ? warp - SW : warp + WARPS - SW) * n_cta;      // of CTA 0
+    Sched sc;
+    int b = 0, w0 = 0, w1 = -1, item = first_item + cta;
+    bool work = false, looked_up = false;
+    auto look_up = [&]() {
+        if ((item >> sh) >= rows_all) return;
+        b = (item >> sh) / p.rows;
+        work = merge_span(b, __ldcg(p.tile_prefix + b), __ldcg(p.tile_prefix + b + 1), sc, w0, w1);
+    };
+    if (p.fused && warp >= SW) {
+        looked_up = __shfl_sync(0xffffffffu, lane == 0 && load_acquire(p.status + SYNC_PREFIX) > 0, 0);
+        if (looked_up) {
+            sc = make_sched(__ldcg(p.tile_prefix + p.batch), p.batch, G, p.seq_units);
+            look_up();
+        }
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == C::QK_WARP) { tc_fence_after(); tmem_dealloc(tmem, C::TMEM_COLS); }
     if (p.fused) {
-        // Merge of the partials by the same launch: grid-wide barrier (the launch is cooperative), then the query rows are
-        // dealt out to all warps - whole rows, halves or quarters, so that every warp has one item at most where there are
-        // few.  A second kernel cost 5 us and more per call (launch, drain, cold code), a third of the small shapes.
-        // What a warp's first item consists of is worked out between arriving at the barrier and waiting for it.
-        const int n_cta = (int)(gridDim.x * gridDim.y), rows_all = p.batch * p.rows, n_warps = n_cta * (C::THREADS / 32);
-        if (tid == 0) red_release(p.status + SYNC_ARRIVE, 1);     // after the __syncthreads: covers the stores of the whole CTA
-        const int sh = rows_all * 4 <= n_warps ? 2 : (rows_all * 2 <= n_warps ? 1 : 0);
-        int it = warp * n_cta + (int)(blockIdx.y * gridDim.x + blockIdx.x);
-        if (lane == 0) grid_wait(p.status + SYNC_PREFIX, 1, abort_flag);
-        __syncwarp();
-        const Sched sc = make_sched(__ldcg(p.tile_prefix + p.batch), p.batch, G, p.seq_units);
-        int row = it >> sh, b = row / p.rows, w0 = 0, w1 = -1, exited = 0;
-        bool work = false;
-        if (row < rows_all) work = merge_span(b, __ldcg(p.tile_prefix + b), __ldcg(p.tile_prefix + b + 1), sc, w0, w1);
-        if (tid == 0) grid_wait(p.status + SYNC_ARRIVE, n_cta, abort_flag);
-        __syncthreads();                                          // also: every warp has seen SYNC_PREFIX
-        if (tid == 0) exited = atomicAdd(p.status + SYNC_EXIT, 1);        // looked at after the merge
-        while (row < rows_all) {
-            if (work) {
-                const int r = row - b * p.rows, d = lane * 4;
-                if (sh == 2) merge_row<1, 12>(p, b, r, w0, w1, (it & 3) * 128 + d);
-                else if (sh == 1) merge_row<2, 4>(p, b, r, w0, w1, (it & 1) * 256 + d);
-                else merge_row<4, 4>(p, b, r, w0, w1, d);
+        int exited = 0;
+        if (tid == 0) {                                           // after the __syncthreads: covers the stores of the whole CTA
+            int* arrive = p.status + SYNC_ARRIVE;
+            const int seen = add_acq_rel(arrive, 1);
+            const bool last = (seen & 0xffff) == n_cta - 1;
+            bool all = last || count_reached(arrive, n_cta, p.meet_cycles);
+            if (!all) {
+                atomicOr(p.status + SYNC_LEFT + (cta >> 5), 1 << (cta & 31));
+                all = (add_acq_rel(arrive, 1 << 16) & 0xffff) == n_cta;
             }
-            it += n_warps;
-            row = it >> sh;
-            if (row >= rows_all) break;
-            b = row / p.rows;
-            work = merge_span(b, __ldcg(p.tile_prefix + b), __ldcg(p.tile_prefix + b + 1), sc, w0, w1);
+            ms.meet = !all ? MEET_LEAVE : (last && seen >> 16 ? MEET_OTHERS : MEET_ALL);
+            if (ms.meet == MEET_OTHERS) {
+                for (int i = 0; i < SYNC_LEFT_WORDS; ++i) ms.left[i] = __ldcg(p.status + SYNC_LEFT + i);
+                __threadfence();
+            }
         }
-        if (tid == 0 && exited == n_cta - 1) {                    // the last one past the barrier: nobody looks at these any more
+        __syncthreads();
+        if (tid == 0) exited = atomicAdd(p.status + SYNC_EXIT, 1);        // looked at after the merge
+        if (ms.meet != MEET_LEAVE) {
+            if (!looked_up) {
+                sc = make_sched(__ldcg(p.tile_prefix + p.batch), p.batch, G, p.seq_units);
+                look_up();
+            }
+            for (int next = 0;;) {
+                for (; (item >> sh) < rows_all; item += n_warps, look_up()) {
+                    if (!work) continue;
+                    const int r = (item >> sh) - b * p.rows, d = lane * 4;
+                    if (sh == 2) merge_row<1, 12>(p, b, r, w0, w1, (item & 3) * 128 + d);
+                    else if (sh == 1) merge_row<2, 4>(p, b, r, w0, w1, (item & 1) * 256 + d);
+                    else merge_row<4, 4>(p, b, r, w0, w1, d);
+                }
+                if (ms.meet != MEET_OTHERS) break;
+                while (next < n_cta && !(ms.left[next >> 5] >> (next & 31) & 1)) ++next;      // those that have left
+                if (next >= n_cta) break;
+                item = first_item + next++;
+                look_up();
+            }
+        }
+        if (tid == 0 && exited == n_cta - 1) {                    // the last one past the meeting: nobody looks at these any more
             p.status[SYNC_AMAX] = 0; p.status[SYNC_AMAX_COUNT] = 0; p.status[SYNC_PREFIX] = 0; p.status[SYNC_ARRIVE] = 0; p.status[SYNC_EXIT] = 0;
+            for (int i = 0; i < SYNC_LEFT_WORDS; ++i) p.status[SYNC_LEFT + i] = 0;
         }
     }
     if (tid == 0 && ms.abort_flag) report_status(p.status, ST_TIMEOUT);
@@ -1192,17 +1250,7 @@ cudaError_t launch_cfg(const MlaParams& p, cudaStream_t stream) {
     const sm100::Maps* maps = nullptr;
     const char* off = getenv("B200_MLA_DISABLE_TMA");                 // testing aid: "1" keeps every tile on the copy loop
     if (KVFMT == KV_E4M3 && !(off && off[0] == '1')) maps = cache_maps(p);
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeCooperative;
-    attr.val.cooperative = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.num_ctas, p.rows / N);
-    cfg.blockDim = dim3(C::THREADS);
-    cfg.dynamicSmemBytes = C::SMEM;
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = p.fused ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, p, maps ? *maps : no_maps, maps != nullptr);
+    return launch_pdl(kernel, dim3(p.num_ctas, p.rows / N), C::THREADS, C::SMEM, stream, p, maps ? *maps : no_maps, maps != nullptr);
 }
 
 template <int KVFMT>

@@ -90,16 +90,23 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, const uint4& v) {
 __device__ __forceinline__ void red_release(int* counter, int v) {
     asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(counter), "r"(v) : "memory");
 }
-// Wait of one thread until the counter in global memory has reached `total`; bounded like mbar_wait.
-__device__ __forceinline__ void grid_wait(const int* counter, int total, volatile int* abort_flag) {
+__device__ __forceinline__ int add_acq_rel(int* counter, int v) {
+    int old;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(counter), "r"(v) : "memory");
+    return old;
+}
+__device__ __forceinline__ int load_acquire(const int* p) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+// One thread looks at a counter (lower 16 bits) in global memory until it has reached `total`, for at most `cycles`.
+__device__ __forceinline__ bool count_reached(const int* counter, int total, int cycles) {
     const long long t0 = clock64();
-    for (;;) {
-        int v;
-        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-        if (v >= total || *abort_flag) return;
-        if (clock64() - t0 > WAIT_LIMIT_CYCLES) break;
-    }
-    *abort_flag = 1;
+    do {
+        if ((load_acquire(counter) & 0xffff) >= total) return true;
+    } while (clock64() - t0 < cycles);
+    return false;
 }
 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }

@@ -701,7 +701,7 @@ def main():
                "sample": f"median of {args.cpu_reps} full {args.workload} calls ({t_cpu * 1e3:.1f} ms each)",
                "us_per_call": t_cpu * 1e6}
 
-    # the tcgen05 path is one cooperative launch (maximum of Q, decode, merge); the warp-level kernel has a combine kernel
+    # the tcgen05 path is one launch (maximum of Q, decode, merge); the warp-level kernel has a combine kernel
     # beside it and, for an FP8-cast Q, an amax kernel; split-KV ranks quantise Q ahead (amax + cast)
     if args.kernel == "generic":
         launches_per_step = 2 + (1 if w["q_format"] == "fp8" else 0)

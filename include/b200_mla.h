@@ -145,7 +145,8 @@ int64_t b200_mla_workspace_bytes(int32_t batch, int32_t heads, int32_t q_len);
 
 /*
  * Split-KV decode: stage 1 (partial attention per KV span) and the log-sum-exp combine, enqueued on `stream` as one
- * cooperative launch where the grid is resident at once, else as two kernels.
+ * launch where the GPU holds the grid at once, else as two kernels.  The launch may be placed while the kernel before it in the
+ * stream drains; it reads and writes nothing before that one is complete.
  * Replaces mla_decode_fwd / mla_decode_stage1_asm_fwd + mla_reduce_v1
  * (mixed-mla/asm_dumps/aiter_mla.py:149-470), the Triton pair _mla_mxfp4_stage1 / _mla_mxfp4_reduce
  * (mixed-mla/submission.py:122-294) and the work-list builder get_mla_metadata_v1

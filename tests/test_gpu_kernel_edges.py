@@ -121,6 +121,47 @@ def test_lengths_around_units_and_tiles(pkg, kv_format, q_format, heads, q_len):
         assert_close(_run(pkg, data, kv_format, q_format, impl="tcgen05", max_ctas=max_ctas), want, tight=1.5e-2)
 
 
+# CTAs that do not wait for one another (0 cycles): each finds the maximum of Q itself, and the last one to arrive merges for all.
+@pytest.mark.parametrize("kv_format,q_format,heads,lens", [("fp8", "fp8", 16, [900, 0, 97, 2000]), ("mxfp4", "bf16", 32, [4000]),
+                                                           ("hybrid", "fp8", 128, [700, 1500, 64]), ("fp8", "bf16", 16, [130] * 300)])
+def test_ctas_that_leave_before_the_merge(pkg, monkeypatch, kv_format, q_format, heads, lens):
+    data = pkg.generate_input(len(lens), 1, max(lens), seed=heads, kv_lens=lens, shuffle_pages=True, num_heads=heads, formats=(kv_format,))
+    want = _run(pkg, data, kv_format, q_format, impl="tcgen05")
+    for cycles in ("0", "300", "0"):                             # none, some, none: and the words they meet at are zero afterwards
+        monkeypatch.setenv("B200_MLA_MEET_CYCLES", cycles)
+        assert torch.equal(_run(pkg, data, kv_format, q_format, impl="tcgen05"), want)
+    monkeypatch.delenv("B200_MLA_MEET_CYCLES")
+    assert torch.equal(_run(pkg, data, kv_format, q_format, impl="tcgen05", check_status=True), want)
+
+
+@pytest.mark.parametrize("kv_format,q_format", [("fp8", "fp8"), ("mxfp4", "bf16")])
+def test_decode_behind_other_work_of_the_stream(pkg, kv_format, q_format):
+    """Its CTAs are placed while the kernel before them drains: what that kernel writes has to be seen, in a graph too."""
+    lens = [3000, 17, 900, 64]
+    sets = [pkg.generate_input(4, 1, 3000, seed=s, kv_lens=lens, shuffle_pages=True, formats=(kv_format,)) for s in (1, 2)]
+    want = [_run(pkg, d, kv_format, q_format) for d in sets]
+    torch.cuda.synchronize()
+    q, planes, table = sets[0][0].clone(), tuple(t.clone() for t in sets[0][1][kv_format]), sets[0][4]["kv_indices"].clone()
+    data = (q, {kv_format: planes}, *sets[0][2:4], dict(sets[0][4], kv_indices=table))
+
+    def step(i):
+        for to, new in zip(planes, sets[i][1][kv_format]):
+            to.view(torch.uint8).copy_(new.view(torch.uint8))
+        table.copy_(sets[i][4]["kv_indices"])
+        q.copy_(sets[i][0])
+        return _run(pkg, data, kv_format, q_format)
+
+    outs = [step(i & 1) for i in range(10)]
+    assert all(torch.equal(o, want[i & 1]) for i, o in enumerate(outs))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        outs = [step(i & 1) for i in range(4)]
+    for _ in range(3):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, want[i & 1]) for i, o in enumerate(outs))
+
+
 # The span search gives a lane ceil(batch / 32) sequences and looks inside them 32 at a time.
 @pytest.mark.parametrize("batch", [31, 32, 33, 64, 65, 300, 1025])
 def test_batches_around_the_lanes_of_the_span_search(pkg, batch):
