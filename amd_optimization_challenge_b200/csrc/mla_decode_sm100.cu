@@ -64,7 +64,8 @@ struct Misc {
     unsigned int q_red[8];                // cross-warp maximum of a split Q
     long long q_off[4];                   // element offset of each 16-row chunk of this row group inside a sequence's Q
     __align__(16) int tile_exp[NS_MAX][8];    // exponent frame of each unit of the tile in each stage
-    __align__(16) float nm[2][2][32];     // P_SCALE_LOG2 - reference maximum per query row: [warpgroup][double buffer][row]
+    __align__(16) float nm[2][2][32];     // P_SCALE_LOG2 - reference maximum per query row, 0 before the first tile: [warpgroup][double buffer][row]
+    __align__(16) float shift[2][32];     // what nm moves by at a tile
     __align__(16) float fac[2][32];       // per-row factors published to a warpgroup
     __align__(16) float red[2][4][32];    // cross-warp column reductions
 };
@@ -91,8 +92,9 @@ struct Cfg {
     // A probability p (relative to the reference maximum) is stored as 2^P_SCALE_LOG2 p; a score more than RECENTER log2 units above
     // the reference maximum moves it.  2^(P_SCALE_LOG2 + RECENTER) must stay below 448.  The smallest step of the stored pair is
     // 2^-13 with lo / 16 in columns of its own, 2^-9 where lo shares hi's columns (MERGED): there the larger factor keeps the same
-    // 2^-17 below the reference maximum, at the price of moving it more often (48 ragged sequences of 128 heads: 85.6 us; with
-    // 2^4 74.7, but like keys 12 binades down came out 28 % wrong).  Block-scaled caches at 64 rows keep 2^4, i.e. 2^-13.
+    // 2^-17 below the reference maximum, at the price of moving it at most tiles (48 ragged sequences of 128 heads: 81 us; 85 when
+    // O was rescaled before the probabilities were computed, all of it, and the scores read three times; less with 2^4, but like
+    // keys 12 binades down come out 28 % wrong).  Block-scaled caches at 64 rows keep 2^4, i.e. 2^-13.
     static constexpr bool DEEP = MERGED && !XF;
     static constexpr float P_SCALE_LOG2 = DEEP ? 8.0f : 4.0f, RECENTER = DEEP ? 0.75f : 4.0f;
     static constexpr int P_CHUNK_BYTES = TILE * 16;               // 16 columns x TILE tokens
@@ -271,14 +273,15 @@ struct Walk {
 // Column reductions over the 32 lanes of a warp by recursive halving: every step exchanges half of the columns that are
 // left, so NC columns cost NC - 1 shuffles (+ 1 for 16) instead of 5 NC.  Lane l ends with column l (NC = 32) or l / 2 (NC = 16).
 template <int NC, bool IS_MAX>
-__device__ __forceinline__ float fold_columns(float (&v)[NC], int lane) {
+__device__ __forceinline__ float fold_columns(const float (&x)[NC], int lane) {
+    float v[NC / 2];
 #pragma unroll
     for (int h = NC / 2, m = 16; h >= 1; h >>= 1, m >>= 1) {
         const bool up = (lane & m) != 0;
 #pragma unroll
         for (int i = 0; i < h; ++i) {
-            const float send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
-            const float got = __shfl_xor_sync(0xffffffffu, send, m);
+            const float a = h == NC / 2 ? x[i] : v[i], b = h == NC / 2 ? x[i + h] : v[i + h];
+            const float got = __shfl_xor_sync(0xffffffffu, up ? a : b, m), keep = up ? b : a;
             v[i] = IS_MAX ? fmaxf(keep, got) : keep + got;
         }
     }
@@ -381,9 +384,12 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
         mbar_init(&ms.o_free, SW);
         ms.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    } else if (tid == 32 * (SW + 1) && use_tma) {
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.lat) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.rope) : "memory");
+    } else if (warp == SW + 1) {
+        ms.nm[0][0][lane] = ms.nm[1][0][lane] = 0.0f;
+        if (lane == 0 && use_tma) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.lat) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.rope) : "memory");
+        }
     }
     __syncwarp();
     pdl_wait();
@@ -601,6 +607,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                             const float sum = (ms.red[sg][0][tok] + ms.red[sg][1][tok]) + (ms.red[sg][2][tok] + ms.red[sg][3][tok]);
                             ms.fac[sg][tok] = sum > 0.0f ? __fdividef(out_scale, sum) : 0.0f;
                             const float lse = sum > 0.0f ? (log2f(sum) - ms.nm[sg][nm_cur][tok]) * LN2 : -INFINITY;
+                            ms.nm[sg][nm_cur][tok] = 0.0f;
                             if (!whole) p.part_lse[orow0 + tok] = lse;
                             else if (p.out_lse) p.out_lse[orow0 + tok] = lse;
                         }
@@ -665,8 +672,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                 const float a_rope = qk_base * kv_tensor_scale;
                 const uint32_t s_addr = tmem + lane_base + sb * C::SC + col0;
                 float x[NC];
-                // x = score in log2 units (+ nm if given: then it is the exponent of the stored probability).  The scores are
-                // not kept beyond that: the rare re-centering path reads them again (the S buffer is handed back after it).
+                // x = score in log2 units + nm: the exponent of the stored probability
                 auto load_scores = [&](const float* nm) {
                     const f32x2 al = pk2(a_lat, a_lat), ar = pk2(a_rope, a_rope), c16 = pk2(0.0625f, 0.0625f);
 #pragma unroll
@@ -681,7 +687,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                         tmem_wait_ld();
 #pragma unroll
                         for (int c = 0; c < 16; c += 4) {
-                            const float4 n4 = nm ? *reinterpret_cast<const float4*>(nm + c0 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                            const float4 n4 = *reinterpret_cast<const float4*>(nm + c0 + c);
 #pragma unroll
                             for (int h = 0; h < 4; h += 2) {
                                 f32x2 lat = pk2(v[c + h], v[c + h + 1]);
@@ -705,12 +711,19 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                         for (int c = 0; c < NC; ++c) if (pos >= lim[c / 16]) x[c] = -INFINITY;
                     }
                 };
-                bool recenter = first;                                               // a new sequence has no reference maximum yet
+                // x = scores relative to the reference maxima (to zero at a sequence's first tile, see nm); from here on the
+                // tile lives in registers and the S buffer goes back
+                if (active) {
+                    load_scores(ms.nm[sg][nm_cur]);
+                    mask_scores();
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&ms.s_empty[sb]);
+                bool recenter = first;
                 if (!first) {
                     float xm = -INFINITY;
                     if (active) {
-                        load_scores(&ms.nm[sg][nm_cur][0]);
-                        mask_scores();
                         xm = x[0];
 #pragma unroll
                         for (int c = 1; c < NC - 1; c += 2) xm = max3(xm, x[c], x[c + 1]);
@@ -724,58 +737,35 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                     if (first) e_run = e_tile;
                     if (e_tile > e_run) { o_frame = pow2i(e_run - e_tile); e_run = e_tile; }
                 }
-                if (recenter || o_frame != 1.0f) {
-                    if (recenter) {
-                        float top = -INFINITY;
-                        if (active) {
-                            load_scores(nullptr);
-                            mask_scores();
-                            top = fold_columns<NC, true>(x, lane);
-                        }
-                        if (NC == 32 || !(lane & 1)) ms.red[sg][wv][NC == 32 ? lane : lane >> 1] = top;
-                        named_bar_sync(bar_id, 128);
-                        if (tok < NC) {                           // one thread per query row
-                            const float mx = fmaxf(fmaxf(ms.red[sg][0][tok], ms.red[sg][1][tok]), fmaxf(ms.red[sg][2][tok], ms.red[sg][3][tok]));
-                            const float m_old = first ? -INFINITY : C::P_SCALE_LOG2 - ms.nm[sg][nm_cur][tok];     // -inf while the row has seen no key
-                            const float m_new = fmaxf(m_old, mx);
-                            ms.fac[sg][tok] = (m_new == m_old) ? 1.0f : (m_old == -INFINITY ? 0.0f : ex2(m_old - m_new));
-                            ms.nm[sg][nm_cur ^ 1][tok] = C::P_SCALE_LOG2 - m_new;
-                        }
-                        nm_cur ^= 1;
-                        named_bar_sync(bar_id, 128);
-                        if (active) {
-                            load_scores(&ms.nm[sg][nm_cur][0]);
-                            mask_scores();
-                        }
+                unsigned int moved = 0;                           // rows of O to rescale
+                if (recenter) {
+                    const float top = active ? fold_columns<NC, true>(x, lane) : -INFINITY;
+                    if (NC == 32 || !(lane & 1)) ms.red[sg][wv][NC == 32 ? lane : lane >> 1] = top;
+                    named_bar_sync(bar_id, 128);
+                    if (tok < NC) {                               // one thread per query row
+                        const float mx = fmaxf(fmaxf(ms.red[sg][0][tok], ms.red[sg][1][tok]), fmaxf(ms.red[sg][2][tok], ms.red[sg][3][tok]));
+                        const float old = ms.nm[sg][nm_cur][tok];
+                        const float next = mx > (first ? -INFINITY : C::P_SCALE_LOG2) ? old + (C::P_SCALE_LOG2 - mx) : old;
+                        ms.nm[sg][nm_cur ^ 1][tok] = next;
+                        ms.shift[sg][tok] = next - old;           // what the rounded maximum has moved by
+                        ms.fac[sg][tok] = ex2(next - old);
+                    }
+                    nm_cur ^= 1;
+                    named_bar_sync(bar_id, 128);
+#pragma unroll
+                    for (int c = 0; c < NC; c += 4) {
+                        const float4 d4 = *reinterpret_cast<const float4*>(&ms.shift[sg][c]);
+                        x[c] += d4.x; x[c + 1] += d4.y; x[c + 2] += d4.z; x[c + 3] += d4.w;
                     }
                     if (!first) {
-                        // O holds the sequence's earlier tiles once PV(g-1) has completed; nothing else touches it until P(g) is published
-                        if (recenter) {
+                        moved = __ballot_sync(0xffffffffu, lane < NC && ms.shift[sg][lane & (NC - 1)] != 0.0f);
 #pragma unroll
-                            for (int c = 0; c < NC / 2; c += 2) {
-                                const float4 f4 = *reinterpret_cast<const float4*>(&ms.fac[sg][2 * c]);
-                                l_acc[c] = mul2(l_acc[c], pk2(f4.x, f4.y)); l_acc[c + 1] = mul2(l_acc[c + 1], pk2(f4.z, f4.w));
-                            }
+                        for (int c = 0; c < NC / 2; c += 2) {
+                            const float4 f4 = *reinterpret_cast<const float4*>(&ms.fac[sg][2 * c]);
+                            l_acc[c] = mul2(l_acc[c], pk2(f4.x, f4.y)); l_acc[c + 1] = mul2(l_acc[c + 1], pk2(f4.z, f4.w));
                         }
-                        mbar_wait(&ms.p_empty[(g - 1) % P_BUFS], (g - 1) / P_BUFS, abort_flag);
-                        tc_fence_after();
-#pragma unroll 1
-                        for (int jb = 0; jb < 4 * (C::MERGED ? 1 : 2) * (NC / 16); ++jb) {      // rare path: kept small, not unrolled
-                            const int c0 = (jb % (NC / 16)) * 16, blk = jb / (NC / 16);        // O block and, side by side, hi / lo half
-                            float o[16];
-                            const uint32_t addr = tmem + lane_base + C::TMEM_O + blk * N + col0 + c0;
-                            tmem_ld16(addr, o);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int c = 0; c < 16; ++c) o[c] *= recenter ? ms.fac[sg][c0 + c] * o_frame : o_frame;
-                            tmem_st16(addr, o);
-                        }
-                        tmem_wait_st();
                     }
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&ms.s_empty[sb]);      // the scores have been read for the last time
                 uint32_t hi[NC / 4], lo[NC / 4];
                 if (active) {
                     // stored probability = p * 2^P_SCALE_LOG2 * 2^(e_unit - e_run): this token's V bytes are in the frame e_unit, O in e_run
@@ -811,6 +801,33 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                         *reinterpret_cast<uint4*>(pbuf + (N / 16 + q) * C::P_CHUNK_BYTES) = make_uint4(lo[4 * q], lo[4 * q + 1], lo[4 * q + 2], lo[4 * q + 3]);
                     }
                     fence_proxy_async();
+                }
+                if (moved || (o_frame != 1.0f && !first)) {
+                    // O holds the sequence's earlier tiles once PV(g-1) has completed; nothing else touches it until P(g) is published.
+                    // This is the last thing before that, with P already stored: the tensor pipe waits only for the rescaling itself.
+                    // Eight rows of the four blocks at a time, where one of them moved.
+                    mbar_wait(&ms.p_empty[(g - 1) % P_BUFS], (g - 1) / P_BUFS, abort_flag);
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int i = 0; i < (C::MERGED ? 1 : 2) * (NC / 8); ++i) {                 // eight rows and, side by side, hi / lo half
+                        const int r = i % (NC / 8) * 8;
+                        if (o_frame == 1.0f && !(moved >> r & 0xffu)) continue;
+                        const uint32_t addr = tmem + lane_base + C::TMEM_O + i / (NC / 8) * N + col0 + r;
+                        float o[4][8];
+#pragma unroll
+                        for (int blk = 0; blk < 4; ++blk) tmem_ld8(addr + blk * C::OB, o[blk]);
+                        float f[8];
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) f[c] = recenter ? ms.fac[sg][r + c] * o_frame : o_frame;
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int blk = 0; blk < 4; ++blk) {
+#pragma unroll
+                            for (int c = 0; c < 8; ++c) o[blk][c] *= f[c];
+                            tmem_st8(addr + blk * C::OB, o[blk]);
+                        }
+                    }
+                    tmem_wait_st();
                 }
                 tc_fence_before();
                 __syncwarp();

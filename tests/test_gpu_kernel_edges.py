@@ -275,6 +275,32 @@ def test_coherent_tail_far_below_the_maximum(pkg, heads, depth, at):
         assert float((got - want).norm() / want.norm()) <= 2.0 ** (depth - 18) + 2.0 ** -8
 
 
+# Scores that climb along the sequence, for different rows at different tiles, so that reference maxima move and O is rescaled
+# again and again.  Against the warp-level kernel; bf16 outputs and probabilities of about eight bits on either side.
+@pytest.mark.parametrize("kv_format,q_format,heads", [("fp8", "fp8", 16), ("fp8", "bf16", 32), ("fp8", "fp8", 64), ("fp8", "fp8", 128),
+                                                      ("mxfp4", "bf16", 16), ("mxfp4", "bf16", 32), ("mxfp4", "fp8", 64), ("hybrid", "fp8", 128)])
+def test_reference_maxima_that_move_at_most_tiles(pkg, kv_format, q_format, heads):
+    lens, g = [1500, 97, 700], torch.Generator().manual_seed(heads)
+    n = sum(lens)
+    kv = 0.5 * torch.randn(n, 1, 576, generator=g)
+    at = torch.cat([torch.arange(k) for k in lens]).float()
+    for j in range(4):
+        kv[:, 0, 32 * j] = at * (0.5 + j) / 700
+    q = 0.2 * torch.randn(3, heads, 576, generator=g)
+    for h in range(heads):
+        q[:, h, 32 * (h % 4)] = 4.0
+    quantise = {"fp8": pkg.quantize_fp8, "mxfp4": pkg.quantize_mxfp4, "hybrid": pkg.quantize_hybrid}[kv_format]
+    planes, q = quantise(kv.bfloat16().cuda()), q.bfloat16().cuda()
+    qc, qs = pkg.quantize_q_fp8(q) if q_format == "fp8" else (q, None)
+    ip = torch.tensor([0, 1500, 1597, 2297], dtype=torch.int32, device="cuda")
+    run = lambda **kw: pkg.mla_decode(qc, qs, kv_format, planes, ip, sm_scale=1.0, **kw).float()
+    want = run(impl="generic")
+    for max_ctas in (1, 0):                                      # one CTA per row group, and spread out
+        got = run(impl="tcgen05", max_ctas=max_ctas)
+        assert torch.isfinite(got).all()
+        assert float((got - want).norm() / want.norm()) <= 2.0 ** -7
+
+
 def _captured(pkg, data, n=1, stream=None):
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph, stream=stream):
