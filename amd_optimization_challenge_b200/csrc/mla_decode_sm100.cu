@@ -1129,7 +1129,11 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
     // Merge of the partials by the same launch: the CTAs meet, then the query rows are dealt out to all warps - whole rows,
     // halves or quarters, so that every warp has one item at most where there are few.  (A second kernel cost 5 us and more per
     // call: launch, drain, cold code.)  The first items go to the warps that are done before the epilogue: they look up
-    // what theirs consists of while the softmax warps still write (three dependent loads, 2 k cycles behind the meeting before).
+    // what theirs consists of while the softmax warps still write (three loads, 2 k cycles behind the meeting otherwise), so a
+    // row is cut up only as far as there are such warps (MXFP4 32 x 1024: 15.15 us with quarters that softmax warps share, 14.7 with
+    // halves), and the loads of all its partials are in flight together where registers allow: one more round over them costs
+    // 0.5 to 1.3 us (halves, four at a time -> six: MXFP4 32 x 1024 14.7 -> 14.1, e4m3 32 x 4096 24.05 -> 23.65; twenty
+    // quarters: spills, 32.9 us for a rank of eight instead of 31.2).
     // The launch is not cooperative (see MlaParams::meet_cycles): a CTA that has waited meet_cycles for the others leaves its share
     // to the last one to arrive.  Whoever comes last sees who has left: a bit in SYNC_LEFT, then the count in the upper half of
     // SYNC_ARRIVE.  A CTA that learns from that count that all have come after all merges its share too; its bit may have been
@@ -1137,22 +1141,19 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
     constexpr int WARPS = C::THREADS / 32;
     const int n_cta = (int)(gridDim.x * gridDim.y), cta = (int)(blockIdx.y * gridDim.x + blockIdx.x);
     const int rows_all = p.batch * p.rows, n_warps = n_cta * WARPS;
-    const int sh = rows_all * 4 <= n_warps ? 2 : (rows_all * 2 <= n_warps ? 1 : 0);
+    const int n_early = n_cta * (WARPS - SW), sh = rows_all * 4 <= n_early ? 2 : (rows_all * 2 <= n_early ? 1 : 0);
     const int first_item = (warp >= SW ? warp - SW : warp + WARPS - SW) * n_cta;      // of CTA 0
-    Sched sc;
     int b = 0, w0 = 0, w1 = -1, item = first_item + cta;
     bool work = false, looked_up = false;
     auto look_up = [&]() {
         if ((item >> sh) >= rows_all) return;
         b = (item >> sh) / p.rows;
-        work = merge_span(b, __ldcg(p.tile_prefix + b), __ldcg(p.tile_prefix + b + 1), sc, w0, w1);
+        const int tt = __ldcg(p.tile_prefix + p.batch), t0 = __ldcg(p.tile_prefix + b), t1 = __ldcg(p.tile_prefix + b + 1);
+        work = merge_span(b, t0, t1, make_sched(tt, p.batch, G, p.seq_units), w0, w1);
     };
     if (p.fused && warp >= SW) {
         looked_up = __shfl_sync(0xffffffffu, lane == 0 && load_acquire(p.status + SYNC_PREFIX) > 0, 0);
-        if (looked_up) {
-            sc = make_sched(__ldcg(p.tile_prefix + p.batch), p.batch, G, p.seq_units);
-            look_up();
-        }
+        if (looked_up) look_up();
     }
     tc_fence_before();
     __syncthreads();
@@ -1177,16 +1178,13 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
         __syncthreads();
         if (tid == 0) exited = atomicAdd(p.status + SYNC_EXIT, 1);        // looked at after the merge
         if (ms.meet != MEET_LEAVE) {
-            if (!looked_up) {
-                sc = make_sched(__ldcg(p.tile_prefix + p.batch), p.batch, G, p.seq_units);
-                look_up();
-            }
+            if (!looked_up) look_up();
             for (int next = 0;;) {
                 for (; (item >> sh) < rows_all; item += n_warps, look_up()) {
                     if (!work) continue;
                     const int r = (item >> sh) - b * p.rows, d = lane * 4;
                     if (sh == 2) merge_row<1, 12>(p, b, r, w0, w1, (item & 3) * 128 + d);
-                    else if (sh == 1) merge_row<2, 4>(p, b, r, w0, w1, (item & 1) * 256 + d);
+                    else if (sh == 1) merge_row<2, 6>(p, b, r, w0, w1, (item & 1) * 256 + d);
                     else merge_row<4, 4>(p, b, r, w0, w1, d);
                 }
                 if (ms.meet != MEET_OTHERS) break;
