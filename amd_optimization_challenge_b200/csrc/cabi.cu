@@ -72,16 +72,16 @@ int meet_cycles() {
 constexpr int kMaxCtasPerSm = 2;
 inline long long align256(long long x) { return (x + 255) & ~255LL; }
 
-// workspace: [header: status word, barrier words | maxima of Q | tile prefix | partial LSE | partial O]
-struct WsLayout { long long status_off, amax_off, prefix_off, lse_off, o_off, total; };
+// workspace: [header: status word, barrier words | maxima of Q | CTAs of each sequence | partial LSE | partial O]
+struct WsLayout { long long status_off, amax_off, table_off, lse_off, o_off, total; };
 
 WsLayout ws_layout(int batch, int rows, int g_max) {
     WsLayout L;
     const long long slots = (long long)g_max + batch;
     L.status_off = 0;
     L.amax_off = 256;
-    L.prefix_off = L.amax_off + align256(Q_AMAX_PARTS * 4);
-    L.lse_off = L.prefix_off + align256((long long)(batch + 1) * 4);
+    L.table_off = L.amax_off + align256(Q_AMAX_PARTS * 4);
+    L.lse_off = L.table_off + align256((long long)batch * 8);
     L.o_off = L.lse_off + align256(slots * rows * 4);
     L.total = L.o_off + align256(slots * rows * (long long)V_DIM * 4);
     return L;
@@ -184,7 +184,7 @@ int32_t b200_mla_decode(const b200_mla_decode_args* a, void* stream_) {
         return fail(B200_MLA_ERR_WORKSPACE, "workspace of %lld bytes is smaller than the %lld required", (long long)a->workspace_bytes, L.total);
     char* ws = (char*)a->workspace;
     p.status = (int*)(ws + L.status_off);
-    p.tile_prefix = (int*)(ws + L.prefix_off);
+    p.seq_ctas = (int2*)(ws + L.table_off);
     p.part_lse = (float*)(ws + L.lse_off);
     p.part_o = (float*)(ws + L.o_off);
 

@@ -19,9 +19,8 @@ namespace {
 __global__ void __launch_bounds__(128) combine_spans_kernel(const MlaParams p) {
     pdl_wait();
     const int b = blockIdx.x;
-    int w0, w1;
-    if (merge_span(b, p.tile_prefix[b], p.tile_prefix[b + 1], make_sched(p.tile_prefix[p.batch], p.batch, p.num_ctas, p.seq_units), w0, w1))
-        merge_row<1, 4>(p, b, blockIdx.y, w0, w1, threadIdx.x * 4);
+    const int2 ctas = p.seq_ctas[b];
+    if (ctas.x != ctas.y) merge_row<1, 4>(p, b, blockIdx.y, ctas.x, ctas.y, threadIdx.x * 4);
 }
 
 constexpr int GROUP = 8;                // parts whose loads are in flight together: the GPUs of a node

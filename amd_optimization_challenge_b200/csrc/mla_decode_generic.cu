@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(THREADS, 2) mla_decode_generic_kernel(const Ml
     build_tile_prefix(p.kv_indptr, p.batch, TILE, prefix);
     const int TT = prefix[p.batch];
     if (w == 0 && blockIdx.y == 0)
-        for (int i = tid; i <= p.batch; i += THREADS) p.tile_prefix[i] = prefix[i];
+        for (int i = tid; i < p.batch; i += THREADS) p.seq_ctas[i] = seq_span(i, prefix[i], prefix[i + 1], make_sched(TT, p.batch, G, p.seq_units));
     if (TT == 0) return;
     const int t_begin = span_begin(prefix, p.batch, w, G, p.seq_units), t_end = span_begin(prefix, p.batch, w + 1, G, p.seq_units);
     if (t_begin >= t_end) return;

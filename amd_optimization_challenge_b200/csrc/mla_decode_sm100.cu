@@ -203,7 +203,7 @@ __device__ __forceinline__ int warp_scan(int v, int lane) {
 }
 
 template <int TILE>
-__device__ __forceinline__ void find_span(const MlaParams& p, int w, int G, int lane, int (&span)[4], bool write_prefix) {
+__device__ __forceinline__ void find_span(const MlaParams& p, int w, int G, int lane, int (&span)[4], bool write_table) {
     const int batch = p.batch, per = (batch + 31) >> 5;
     const int s0 = min(lane * per, batch), s1 = min(s0 + per, batch);
     int mine = 0;
@@ -238,13 +238,13 @@ __device__ __forceinline__ void find_span(const MlaParams& p, int w, int G, int 
         if (e) t_end = t; else t_first = t;
     }
     span[0] = seq; span[1] = seq_t0; span[2] = t_first; span[3] = t_end;
-    if (write_prefix) {                                           // for the merge
+    if (write_table) {                                            // for the merge
         int t = incl - mine;
         for (int b = s0; b < s1; ++b) {
-            p.tile_prefix[b] = t;
-            t += seq_tiles<TILE>(p.kv_indptr, b, s1);
+            const int n = seq_tiles<TILE>(p.kv_indptr, b, s1);
+            p.seq_ctas[b] = seq_span(b, t, t + n, sc);
+            t += n;
         }
-        if (lane == 0) p.tile_prefix[batch] = tt;
         __syncwarp();
         if (lane == 0 && p.fused) red_release(p.status + SYNC_PREFIX, 1);      // cumulative: __syncwarp orders the lanes' stores before it
     }
@@ -1129,7 +1129,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
     // Merge of the partials by the same launch: the CTAs meet, then the query rows are dealt out to all warps - whole rows,
     // halves or quarters, so that every warp has one item at most where there are few.  (A second kernel cost 5 us and more per
     // call: launch, drain, cold code.)  The first items go to the warps that are done before the epilogue: they look up
-    // what theirs consists of while the softmax warps still write (three loads, 2 k cycles behind the meeting otherwise), so a
+    // what theirs consists of while the softmax warps still write (a load, about 1 k cycles behind the meeting otherwise), so a
     // row is cut up only as far as there are such warps (MXFP4 32 x 1024: 15.15 us with quarters that softmax warps share, 14.7 with
     // halves), and the loads of all its partials are in flight together where registers allow: one more round over them costs
     // 0.5 to 1.3 us (halves, four at a time -> six: MXFP4 32 x 1024 14.7 -> 14.1, e4m3 32 x 4096 24.05 -> 23.65; twenty
@@ -1148,8 +1148,9 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
     auto look_up = [&]() {
         if ((item >> sh) >= rows_all) return;
         b = (item >> sh) / p.rows;
-        const int tt = __ldcg(p.tile_prefix + p.batch), t0 = __ldcg(p.tile_prefix + b), t1 = __ldcg(p.tile_prefix + b + 1);
-        work = merge_span(b, t0, t1, make_sched(tt, p.batch, G, p.seq_units), w0, w1);
+        const int2 ctas = __ldcg(p.seq_ctas + b);
+        w0 = ctas.x; w1 = ctas.y;
+        work = w0 != w1;                                          // one CTA has finished the sequence; none: zeros
     };
     if (p.fused && warp >= SW) {
         looked_up = __shfl_sync(0xffffffffu, lane == 0 && load_acquire(p.status + SYNC_PREFIX) > 0, 0);
