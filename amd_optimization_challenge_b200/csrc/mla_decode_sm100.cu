@@ -28,10 +28,11 @@
 //        1 QK warp, 1 PV warp (the whole warp runs the loop, one elected lane issues), for a block-scaled cache 2 fetch warps
 //        (the PV warp, or the first fetch warp, searches the CTA's span before that)
 // What bounds it, and microseconds a call before (a kernel per family, maximum of Q and merge as launches of their own, one
-// issuing warp) and now: e4m3 256 x 8192 the HBM rate (264 -> 216), 128 heads over an e4m3 cache the chain load -> QK -> softmax -> PV
-// of two stages (236 -> 86), MXFP4 64 x 8192 the same chain with the conversion in it (96 -> 67), MXFP4 8 x 131072 with two
-// queries conversion and shared memory (214 -> 150), hybrid 128 heads the MMA streams (640 -> 395), e4m3 4 x 1024 latencies (23.5 -> 12.3).
-// Synchronisation is mbarrier based; every wait is bounded and on expiry sets a status word.
+// issuing warp) and now: e4m3 256 x 8192 the HBM rate (264 -> 198), 128 heads over an e4m3 cache the chain load -> QK -> softmax -> PV
+// of two stages (236 -> 79), MXFP4 64 x 8192 the same chain with the conversion in it (96 -> 63), MXFP4 8 x 131072 with two
+// queries and hybrid 128 heads shared memory, conversion and MMA operands alike (214 -> 141, 640 -> 382), e4m3 4 x 1024 latencies (23.5 -> 10.0).
+// Synchronisation is mbarrier based; every such wait is bounded and on expiry sets a status word.  The two waits for other CTAs
+// are shorter and need no status: see MlaParams::meet_cycles.
 //
 // Role in the reference: the split-KV stage-1 kernels (mixed-mla/submission.py:122-250,
 // mixed-mla/versions/hip_mxfp4_v5/submission.py:214-656) and their block decode (mixed-mla/triton_mla_mxfp4.py:20-67).
