@@ -43,10 +43,12 @@ __device__ __forceinline__ T load_global(const T* p) { return *p; }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Words of the 256-byte workspace header behind the status word.  ST_FORWARD: address (two words) of a second status word that
-// receives the same bits, 0 if there is none.  SYNC_*: for launches whose CTAs work together; they are zero between launches:
-// the last CTA to exit resets them.  SYNC_LEFT: one bit per CTA.
-enum { ST_FORWARD = 2, SYNC_AMAX = 16, SYNC_AMAX_COUNT = 17, SYNC_PREFIX = 18, SYNC_ARRIVE = 32, SYNC_EXIT = 48, SYNC_LEFT = 52, SYNC_LEFT_WORDS = 8 };
-constexpr int MAX_FUSED_CTAS = 32 * SYNC_LEFT_WORDS;
+// receives the same bits, 0 if there is none.  ST_LEAVES: how many CTAs have left a meeting before all had come, in all launches
+// so far (for tests and measurements).  SYNC_*: for launches whose CTAs work together; they are zero between launches: the last
+// CTA to exit resets them.  SYNC_ARRIVED, SYNC_LEFT: SYNC_MASK_WORDS words each, one bit per CTA.
+enum { ST_FORWARD = 2, ST_LEAVES = 4, SYNC_AMAX = 16, SYNC_AMAX_COUNT = 17, SYNC_PREFIX = 18, SYNC_ARRIVE = 32, SYNC_ARRIVED = 36, SYNC_EXIT = 48,
+       SYNC_LEFT = 52, SYNC_MASK_WORDS = 8 };
+constexpr int MAX_FUSED_CTAS = 32 * SYNC_MASK_WORDS;
 
 struct MlaParams {
     int batch, heads, q_len, rows;      // rows = q_len * heads (query rows per sequence)
@@ -82,7 +84,8 @@ struct MlaParams {
     int fused;                          // the CTAs of the launch also merge the partials, where they meet
     // How long a CTA waits for the others of its launch, twice: for the maximum of Q and before the merge.  They are all resident at
     // once unless something else holds SMs, but nothing depends on it: when the time is up, the CTA looks at all of Q itself, and
-    // leaves its share of the merge to the last CTA to arrive.  So the launch need not be cooperative, and it can overlap with the
+    // merges what it can of its share of the rows; the rest goes to the CTAs that are late, each of which can be left with rows of
+    // the sequences it holds and no others.  So the launch need not be cooperative, and it can overlap with the
     // end of the kernel before it (launch_pdl): 0.8 us between two kernels instead of 2.1, and no rounding up to ticks of 1 or 2 us,
     // which is how other launches of a stream start (e4m3 4 x 1024 12.3 -> 10.0 us a call, 32 x 4096 26.3 -> 23.9).
     int meet_cycles;
@@ -145,9 +148,11 @@ __device__ __forceinline__ void store_bf16x4(__nv_bfloat16* dst, float4 v) {
     *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<uint2*>(o);
 }
 
+// Where partials are and merged rows go (see MlaParams).
+struct MergeIo { const float *part_o, *part_lse; __nv_bfloat16* out; float *out_o_f32, *out_lse; int rows; };
 
-template <int V, int U>
-__device__ __forceinline__ void merge_row(const MlaParams& p, int b, int r, int w0, int w1, int d) {
+template <int V, int U, typename Io>
+__device__ __forceinline__ void merge_row(const Io& p, int b, int r, int w0, int w1, int d) {
     const long long orow = (long long)b * p.rows + r;
     float M = -INFINITY, den = 0.f;
     float4 acc[V];

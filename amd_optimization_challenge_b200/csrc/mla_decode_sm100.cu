@@ -52,7 +52,11 @@ constexpr int RAW_MAX = 10;               // landing buffers of a block-scaled c
 constexpr int SMEM_LIMIT = 232448;        // opt-in shared memory per CTA
 constexpr int E_BIAS = 127 + 6;           // operand bytes of a block-scaled unit are in units of 2^(E_unit - E_BIAS)
 
-enum { MEET_LEAVE = 0, MEET_ALL = 1, MEET_OTHERS = 2 };
+// Outcome of the CTAs' meeting for one of them: bits, all clear where every CTA came in time.  MEET_LEFT: it has left before the last
+// came.  MEET_LATE: others had left before it came.  MEET_NO_TABLE: MlaParams::seq_ctas is not there yet.
+enum { MEET_LEFT = 1, MEET_LATE = 2, MEET_NO_TABLE = 4 };
+constexpr int NO_BIT_CYCLES = 20000;      // 10 us, what the CTAs of an ordinary call are apart: as long a CTA only counts as come
+enum { MASK_ARRIVED = 0, MASK_LATE_ARRIVED = 1, MASK_LATE_LEFT = 2 };      // see Misc::mask
 
 struct Misc {
     uint64_t kv_full[NS_MAX], kv_empty[NS_MAX][4], s_full[2], s_empty[2], p_full[2], p_empty[2], q_full, o_free;
@@ -60,7 +64,7 @@ struct Misc {
     int raw_slot[RAW_MAX][UNIT_TOK];      // cache rows of the unit in each landing buffer
     uint32_t tmem_base;
     int abort_flag;
-    int meet, left[SYNC_LEFT_WORDS];      // outcome of the CTAs' meeting (MEET_*), the CTAs that have left before it
+    int meet;                             // outcome of the CTAs' meeting (MEET_*)
     int span[4];                          // first sequence, its first global tile, first and end tile of this CTA
     unsigned int q_red[8];                // cross-warp maximum of a split Q
     long long q_off[4];                   // element offset of each 16-row chunk of this row group inside a sequence's Q
@@ -69,7 +73,11 @@ struct Misc {
     __align__(16) float shift[2][32];     // what nm moves by at a tile
     __align__(16) float fac[2][32];       // per-row factors published to a warpgroup
     __align__(16) float red[2][4][32];    // cross-warp column reductions
+    // The CTAs that had come when this one left; those that had come, and those that had left, when it came.  In memory that the
+    // fetch warps are done with by then.
+    __device__ __forceinline__ int (&mask(int which))[UNIT_TOK] { return raw_slot[which]; }
 };
+static_assert(SYNC_MASK_WORDS <= UNIT_TOK, "Misc::mask");
 
 template <int N_, int KVFMT, int QFMT>
 struct Cfg {
@@ -203,13 +211,32 @@ __device__ __forceinline__ int warp_scan(int v, int lane) {
     return v;
 }
 
+// The table of the merge, by the lanes of a warp: the CTAs of this lane's sequences [s0, s1), the first of which begins at tile t.
+template <int TILE>
+__device__ __forceinline__ void write_seq_ctas(const MlaParams& p, const Sched& sc, int s0, int s1, int t) {
+    for (int b = s0; b < s1; ++b) {
+        const int n = seq_tiles<TILE>(p.kv_indptr, b, s1);
+        p.seq_ctas[b] = seq_span(b, t, t + n, sc);
+        t += n;
+    }
+    __syncwarp();
+}
+
+// This lane's sequences [s0, s1), and the tiles up to and with them.
+template <int TILE>
+__device__ __forceinline__ int lane_tiles(const MlaParams& p, int lane, int& s0, int& s1, int& mine) {
+    const int per = (p.batch + 31) >> 5;
+    s0 = min(lane * per, p.batch); s1 = min(s0 + per, p.batch);
+    mine = 0;
+    for (int b = s0; b < s1; ++b) mine += seq_tiles<TILE>(p.kv_indptr, b, s1);
+    return warp_scan(mine, lane);
+}
+
 template <int TILE>
 __device__ __forceinline__ void find_span(const MlaParams& p, int w, int G, int lane, int (&span)[4], bool write_table) {
     const int batch = p.batch, per = (batch + 31) >> 5;
-    const int s0 = min(lane * per, batch), s1 = min(s0 + per, batch);
-    int mine = 0;
-    for (int b = s0; b < s1; ++b) mine += seq_tiles<TILE>(p.kv_indptr, b, s1);
-    const int incl = warp_scan(mine, lane);                       // tiles up to and with this lane's sequences
+    int s0, s1, mine;
+    const int incl = lane_tiles<TILE>(p, lane, s0, s1, mine);
     const int tt = __shfl_sync(0xffffffffu, incl, 31);
     const Sched sc = make_sched(tt, batch, G, p.seq_units);
     int t_first = 0, t_end = 0, seq = 0, seq_t0 = 0;
@@ -239,16 +266,65 @@ __device__ __forceinline__ void find_span(const MlaParams& p, int w, int G, int 
         if (e) t_end = t; else t_first = t;
     }
     span[0] = seq; span[1] = seq_t0; span[2] = t_first; span[3] = t_end;
-    if (write_table) {                                            // for the merge
-        int t = incl - mine;
-        for (int b = s0; b < s1; ++b) {
-            const int n = seq_tiles<TILE>(p.kv_indptr, b, s1);
-            p.seq_ctas[b] = seq_span(b, t, t + n, sc);
-            t += n;
-        }
-        __syncwarp();
+    if (write_table) {
+        write_seq_ctas<TILE>(p, sc, s0, s1, incl - mine);
         if (lane == 0 && p.fused) red_release(p.status + SYNC_PREFIX, 1);      // cumulative: __syncwarp orders the lanes' stores before it
     }
+}
+
+// Meeting of the CTAs (end of the kernel).  One thread: the CTAs that have come, every one that had when this began among them, and
+// their partials are visible.  A CTA sets its bit NO_BIT_CYCLES after being counted; the wait is bounded like mbar_wait.
+__device__ __forceinline__ void who_came(int* status, int n_cta, int (&mask)[UNIT_TOK], volatile int* abort_flag) {
+    const long long t0 = clock64();
+    for (;;) {
+        int bits = 0;
+#pragma unroll 1
+        for (int i = 0; i < SYNC_MASK_WORDS; ++i) {
+            const int word = load_acquire(status + SYNC_ARRIVED + i);
+            mask[i] = word;
+            bits += __popc(word);
+        }
+        const int count = load_acquire(status + SYNC_ARRIVE) & 0xffff;
+        if (bits == count) return;
+        if (count == n_cta) break;
+        if (*abort_flag || clock64() - t0 > WAIT_LIMIT_CYCLES) { *abort_flag = 1; break; }
+    }
+    for (int i = 0; i < SYNC_MASK_WORDS; ++i) mask[i] = -1;
+}
+// Whether the CTAs [lo, hi] are all in the mask (true if there are none).
+__device__ __forceinline__ bool in_mask(const int (&mask)[UNIT_TOK], int lo, int hi) {
+    for (int i = lo >> 5; i <= hi >> 5 && lo <= hi; ++i) {
+        const unsigned int want = (i == lo >> 5 ? ~0u << (lo & 31) : ~0u) & (i == hi >> 5 ? ~0u >> (31 - (hi & 31)) : ~0u);
+        if (want & ~(unsigned int)mask[i]) return false;
+    }
+    return true;
+}
+// The first sequence from b0 on that CTA w holds together with others, and its CTAs; p.batch if there is none.
+__device__ __forceinline__ int next_shared(const MlaParams& p, int b0, int w, int lane, int2& ctas) {
+    for (; b0 < p.batch; b0 += 32) {
+        const int2 c = b0 + lane < p.batch ? __ldcg(p.seq_ctas + b0 + lane) : make_int2(0, -1);
+        const unsigned int hit = __ballot_sync(0xffffffffu, c.x < c.y && c.x <= w && w <= c.y);
+        if (hit) {
+            const int l = __ffs(hit) - 1;
+            ctas = make_int2(__shfl_sync(0xffffffffu, c.x, l), __shfl_sync(0xffffffffu, c.y, l));
+            return b0 + l;
+        }
+        if (__ballot_sync(0xffffffffu, c.x > w)) break;
+    }
+    return p.batch;
+}
+
+// One item of the merge: row r of sequence b (sh = 0), a half (1) or a quarter of it (2), which `item` tells.
+template <typename Io>
+__device__ __forceinline__ void merge_item(const Io& io, int b, int r, int w0, int w1, int item, int sh, int lane) {
+    if (sh == 2) merge_row<1, 12>(io, b, r, w0, w1, (item & 3) * 128 + lane * 4);
+    else if (sh == 1) merge_row<2, 6>(io, b, r, w0, w1, (item & 1) * 256 + lane * 4);
+    else merge_row<4, 4>(io, b, r, w0, w1, lane * 4);
+}
+// The same code for CTAs that did not all come in time.  Not inlined: a second copy inside the kernel cost the calls that never reach
+// it registers (4-byte spills; e4m3 32 x 4096 24.15 us, 23.9 so).
+__device__ __noinline__ void merge_item_late(MergeIo io, int b, int r, int w0, int w1, int item, int sh, int lane) {
+    merge_item(io, b, r, w0, w1, item, sh, lane);
 }
 
 // Position of one role inside the CTA's span: the sequence of the current tile and its geometry.
@@ -1135,10 +1211,17 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
     // halves), and the loads of all its partials are in flight together where registers allow: one more round over them costs
     // 0.5 to 1.3 us (halves, four at a time -> six: MXFP4 32 x 1024 14.7 -> 14.1, e4m3 32 x 4096 24.05 -> 23.65; twenty
     // quarters: spills, 32.9 us for a rank of eight instead of 31.2).
-    // The launch is not cooperative (see MlaParams::meet_cycles): a CTA that has waited meet_cycles for the others leaves its share
-    // to the last one to arrive.  Whoever comes last sees who has left: a bit in SYNC_LEFT, then the count in the upper half of
-    // SYNC_ARRIVE.  A CTA that learns from that count that all have come after all merges its share too; its bit may have been
-    // seen, and then both write the same values.
+    // The launch is not cooperative (see MlaParams::meet_cycles): a CTA that has waited meet_cycles for the others goes.  It says so (its
+    // bit in SYNC_LEFT, then one in the upper half of SYNC_ARRIVE), looks who has come, and merges those rows of its share whose
+    // partials are all there.  A row that it has to leave behind lacks a CTA that comes later.  That one learns from SYNC_ARRIVE that
+    // others had left, and the last CTA of a sequence to come merges what those have left of it.  So what falls on a late CTA is rows of the
+    // one or two sequences that it shares with others, in its row group: 64 rows of 74 partials at most, 10 MB.  When all of it fell on the last
+    // CTA of the call, 50 us of waiting in vain became several hundred of merging by one CTA (us a call: 500 sequences of 3 tokens, 500 of 700
+    // and 20 of 100000 in turn, 128 heads over an e4m3 cache, 1447, 872 so and 937 if every CTA waits for all; 3000 of 5 and 30 of 300000,
+    // MXFP4, 2315, 1115 and 1162; 48 sequences of 128 heads with a limit of 0, 753 and 90, where 78 is without anyone leaving).
+    // Two that write a row (a CTA that learns only as it goes that all have come merges its share after all) write the same values.
+    // Who has come is read from SYNC_ARRIVED, whose bits are set after the count: a look that shows as many bits as the count
+    // read after it shows every CTA that had come by then.
     constexpr int WARPS = C::THREADS / 32;
     const int n_cta = (int)(gridDim.x * gridDim.y), cta = (int)(blockIdx.y * gridDim.x + blockIdx.x);
     const int rows_all = p.batch * p.rows, n_warps = n_cta * WARPS;
@@ -1164,41 +1247,76 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
         int exited = 0;
         if (tid == 0) {                                           // after the __syncthreads: covers the stores of the whole CTA
             int* arrive = p.status + SYNC_ARRIVE;
+            const int bit = 1 << (cta & 31);
             const int seen = add_acq_rel(arrive, 1);
-            const bool last = (seen & 0xffff) == n_cta - 1;
-            bool all = last || count_reached(arrive, n_cta, p.meet_cycles);
-            if (!all) {
-                atomicOr(p.status + SYNC_LEFT + (cta >> 5), 1 << (cta & 31));
-                all = (add_acq_rel(arrive, 1 << 16) & 0xffff) == n_cta;
+            bool all = (seen & 0xffff) == n_cta - 1;
+            int meet = 0;
+            if (!all && !(seen >> 16)) all = count_reached(arrive, n_cta, min(p.meet_cycles, NO_BIT_CYCLES));
+            if (__builtin_expect(!all || seen >> 16, 0)) {
+                or_release(p.status + SYNC_ARRIVED + (cta >> 5), bit);
+                if (seen >> 16) {
+                    meet = MEET_LATE;
+                    who_came(p.status, n_cta, ms.mask(MASK_LATE_ARRIVED), abort_flag);
+                    for (int i = 0; i < SYNC_MASK_WORDS; ++i) ms.mask(MASK_LATE_LEFT)[i] = load_acquire(p.status + SYNC_LEFT + i);
+                }
+                if (!all) all = count_reached(arrive, n_cta, p.meet_cycles);
+                if (!all) {
+                    atomicOr(p.status + SYNC_LEFT + (cta >> 5), bit);
+                    all = (add_acq_rel(arrive, 1 << 16) & 0xffff) == n_cta;
+                }
+                if (!all) {
+                    meet |= MEET_LEFT;
+                    who_came(p.status, n_cta, ms.mask(MASK_ARRIVED), abort_flag);
+                    atomicAdd(p.status + ST_LEAVES, 1);
+                }
+                if (meet && load_acquire(p.status + SYNC_PREFIX) == 0) meet |= MEET_NO_TABLE;
             }
-            ms.meet = !all ? MEET_LEAVE : (last && seen >> 16 ? MEET_OTHERS : MEET_ALL);
-            if (ms.meet == MEET_OTHERS) {
-                for (int i = 0; i < SYNC_LEFT_WORDS; ++i) ms.left[i] = __ldcg(p.status + SYNC_LEFT + i);
-                __threadfence();
-            }
+            ms.meet = meet;
         }
         __syncthreads();
         if (tid == 0) exited = atomicAdd(p.status + SYNC_EXIT, 1);        // looked at after the merge
-        if (ms.meet != MEET_LEAVE) {
+        const int meet = ms.meet;
+        if (__builtin_expect(meet == 0, 1)) {
             if (!looked_up) look_up();
-            for (int next = 0;;) {
-                for (; (item >> sh) < rows_all; item += n_warps, look_up()) {
-                    if (!work) continue;
-                    const int r = (item >> sh) - b * p.rows, d = lane * 4;
-                    if (sh == 2) merge_row<1, 12>(p, b, r, w0, w1, (item & 3) * 128 + d);
-                    else if (sh == 1) merge_row<2, 6>(p, b, r, w0, w1, (item & 1) * 256 + d);
-                    else merge_row<4, 4>(p, b, r, w0, w1, d);
+            for (; (item >> sh) < rows_all; item += n_warps, look_up())
+                if (work) merge_item(p, b, (item >> sh) - b * p.rows, w0, w1, item, sh, lane);
+        } else {
+            if (meet & MEET_NO_TABLE) {                           // the first CTA has not begun: the same table, by this one
+                if (warp == 0) {
+                    int s0, s1, mine;
+                    const int incl = lane_tiles<TILE>(p, lane, s0, s1, mine);
+                    write_seq_ctas<TILE>(p, make_sched(__shfl_sync(0xffffffffu, incl, 31), p.batch, G, p.seq_units), s0, s1, incl - mine);
                 }
-                if (ms.meet != MEET_OTHERS) break;
-                while (next < n_cta && !(ms.left[next >> 5] >> (next & 31) & 1)) ++next;      // those that have left
-                if (next >= n_cta) break;
-                item = first_item + next++;
+                __syncthreads();
+            }
+            look_up();
+            int end = rows_all << sh, heir_of = -1;               // >= 0: rows that others have left of this sequence
+            for (;;) {
+                for (; item < end; item += heir_of < 0 ? n_warps : WARPS, look_up()) {
+                    if (!work) continue;
+                    const int r = (item >> sh) - b * p.rows, y = r / N;
+                    if (heir_of >= 0 ? in_mask(ms.mask(MASK_LATE_LEFT), item % n_cta, item % n_cta)
+                                     : !(meet & MEET_LEFT) || in_mask(ms.mask(MASK_ARRIVED), y * G + w0, y * G + w1))
+                        merge_item_late(MergeIo{p.part_o, p.part_lse, p.out, p.out_o_f32, p.out_lse, p.rows}, b, r, w0, w1, item, sh, lane);
+                }
+                if (!(meet & MEET_LATE)) break;
+                int2 ctas;                                        // the next sequence that this CTA shares with others
+                if (heir_of < 0) heir_of = ms.span[0] - 1;
+                do heir_of = next_shared(p, heir_of + 1, (int)blockIdx.x, lane, ctas);
+                while (heir_of < p.batch && !in_mask(ms.mask(MASK_LATE_ARRIVED), blockIdx.y * G + ctas.x, blockIdx.y * G + ctas.y));
+                if (heir_of >= p.batch) break;
+                item = heir_of * p.rows + (int)blockIdx.y * N;
+                end = (item + N) << sh;
+                item = (item << sh) + warp;
                 look_up();
             }
         }
         if (tid == 0 && exited == n_cta - 1) {                    // the last one past the meeting: nobody looks at these any more
             p.status[SYNC_AMAX] = 0; p.status[SYNC_AMAX_COUNT] = 0; p.status[SYNC_PREFIX] = 0; p.status[SYNC_ARRIVE] = 0; p.status[SYNC_EXIT] = 0;
-            for (int i = 0; i < SYNC_LEFT_WORDS; ++i) p.status[SYNC_LEFT + i] = 0;
+            for (int i = 0; i < SYNC_MASK_WORDS; i += 4) {
+                *reinterpret_cast<int4*>(p.status + SYNC_ARRIVED + i) = make_int4(0, 0, 0, 0);
+                *reinterpret_cast<int4*>(p.status + SYNC_LEFT + i) = make_int4(0, 0, 0, 0);
+            }
         }
     }
     if (tid == 0 && ms.abort_flag) report_status(p.status, ST_TIMEOUT);

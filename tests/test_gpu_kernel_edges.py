@@ -121,17 +121,64 @@ def test_lengths_around_units_and_tiles(pkg, kv_format, q_format, heads, q_len):
         assert_close(_run(pkg, data, kv_format, q_format, impl="tcgen05", max_ctas=max_ctas), want, tight=1.5e-2)
 
 
-# CTAs that do not wait for one another (0 cycles): each finds the maximum of Q itself, and the last one to arrive merges for all.
+def _run_over_nans(pkg, data, kv_format, q_format, **more):
+    """_run whose output block holds NaNs before the call: a row that nobody writes is seen."""
+    block = torch.full((data[0].shape[0], data[0].shape[1], 512), float("nan"), dtype=torch.bfloat16, device="cuda")
+    at = block.data_ptr()
+    del block
+    out = _run(pkg, data, kv_format, q_format, **more)
+    assert out.data_ptr() == at
+    return out
+
+
+def _left(pkg):
+    """CTAs that have left a meeting of eager calls before all had come (word 4 of the workspaces)."""
+    from amd_optimization_challenge_b200 import submission
+    return sum(int(ws[16:20].view(torch.int32)) for ws in submission._workspace_cache.values())
+
+
+# CTAs that do not wait for one another (0 cycles), or not for long: each finds the maximum of Q itself, and those that are late
+# merge what the others had to leave behind.
 @pytest.mark.parametrize("kv_format,q_format,heads,lens", [("fp8", "fp8", 16, [900, 0, 97, 2000]), ("mxfp4", "bf16", 32, [4000]),
-                                                           ("hybrid", "fp8", 128, [700, 1500, 64]), ("fp8", "bf16", 16, [130] * 300)])
+                                                           ("hybrid", "fp8", 128, [700, 1500, 64]), ("fp8", "bf16", 16, [130] * 300),
+                                                           ("fp8", "fp8", 128, [3] * 150 + [6000, 0, 9000] + [3] * 150)])
 def test_ctas_that_leave_before_the_merge(pkg, monkeypatch, kv_format, q_format, heads, lens):
     data = pkg.generate_input(len(lens), 1, max(lens), seed=heads, kv_lens=lens, shuffle_pages=True, num_heads=heads, formats=(kv_format,))
     want = _run(pkg, data, kv_format, q_format, impl="tcgen05")
-    for cycles in ("0", "300", "0"):                             # none, some, none: and the words they meet at are zero afterwards
-        monkeypatch.setenv("B200_MLA_MEET_CYCLES", cycles)
-        assert torch.equal(_run(pkg, data, kv_format, q_format, impl="tcgen05"), want)
+    assert torch.isfinite(want).all()
+    for cycles in (0, 300, 0, 1000, 2000, 4000, 6000, 8000, 12000, 20000, 0):     # up to the time that they are apart
+        monkeypatch.setenv("B200_MLA_MEET_CYCLES", str(cycles))
+        before = _left(pkg)
+        for _ in range(5):
+            assert torch.equal(_run_over_nans(pkg, data, kv_format, q_format, impl="tcgen05"), want)
+        assert cycles or _left(pkg) > before
     monkeypatch.delenv("B200_MLA_MEET_CYCLES")
-    assert torch.equal(_run(pkg, data, kv_format, q_format, impl="tcgen05", check_status=True), want)
+    # and the words they meet at are zero afterwards
+    assert torch.equal(_run_over_nans(pkg, data, kv_format, q_format, impl="tcgen05", check_status=True), want)
+
+
+# What CTAs leave behind must not all fall on one of them: these calls took ten times as long then.
+@pytest.mark.parametrize("kv_format,q_format", [("fp8", "bf16")])
+def test_a_call_whose_ctas_leave_takes_little_longer(pkg, monkeypatch, kv_format, q_format):
+    data = pkg.generate_input(24, 1, 3000, seed=3, kv_lens=[3000] * 24, num_heads=128, formats=(kv_format,))
+
+    def us(n=20):
+        times = []
+        for _ in range(5):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda._sleep(2_000_000)
+            start.record()
+            for _ in range(n):
+                _run(pkg, data, kv_format, q_format)
+            end.record()
+            torch.cuda.synchronize()
+            times.append(start.elapsed_time(end) * 1e3 / n)
+        return min(times)
+
+    waiting = us()
+    monkeypatch.setenv("B200_MLA_MEET_CYCLES", "0")
+    leaving = us()
+    assert leaving <= 3 * waiting, f"{leaving:.0f} us, {waiting:.0f} us where CTAs wait"
 
 
 @pytest.mark.parametrize("kv_format,q_format", [("fp8", "fp8"), ("mxfp4", "bf16")])
