@@ -45,8 +45,8 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // Words of the 256-byte workspace header behind the status word.  ST_FORWARD: address (two words) of a second status word that
 // receives the same bits, 0 if there is none.  ST_LEAVES: how many CTAs have left a meeting before all had come, in all launches
 // so far (for tests and measurements).  SYNC_*: for launches whose CTAs work together; they are zero between launches: the last
-// CTA to exit resets them.  SYNC_ARRIVED, SYNC_LEFT: SYNC_MASK_WORDS words each, one bit per CTA.
-enum { ST_FORWARD = 2, ST_LEAVES = 4, SYNC_AMAX = 16, SYNC_AMAX_COUNT = 17, SYNC_PREFIX = 18, SYNC_ARRIVE = 32, SYNC_ARRIVED = 36, SYNC_EXIT = 48,
+// CTA to exit resets them.  SYNC_AMAX_DONE, SYNC_ARRIVED, SYNC_LEFT: SYNC_MASK_WORDS words each, one bit per CTA.
+enum { ST_FORWARD = 2, ST_LEAVES = 4, SYNC_AMAX = 16, SYNC_AMAX_COUNT = 17, SYNC_PREFIX = 18, SYNC_AMAX_DONE = 20, SYNC_ARRIVE = 32, SYNC_ARRIVED = 36, SYNC_EXIT = 48,
        SYNC_LEFT = 52, SYNC_MASK_WORDS = 8 };
 constexpr int MAX_FUSED_CTAS = 32 * SYNC_MASK_WORDS;
 
@@ -83,8 +83,8 @@ struct MlaParams {
                                         //   or, nullptr, from the maximum the CTAs of the launch find together (SYNC_AMAX)
     int fused;                          // the CTAs of the launch also merge the partials, where they meet
     // How long a CTA waits for the others of its launch, twice: for the maximum of Q and before the merge.  They are all resident at
-    // once unless something else holds SMs, but nothing depends on it: when the time is up, the CTA looks at all of Q itself, and
-    // merges what it can of its share of the rows; the rest goes to the CTAs that are late, each of which can be left with rows of
+    // once unless something else holds SMs, but nothing depends on it: when the time is up, the CTA looks at shares of Q that
+    // nobody has looked at yet, and merges what it can of its share of the rows; the rest goes to the CTAs that are late, each of which can be left with rows of
     // the sequences it holds and no others.  So the launch need not be cooperative, and it can overlap with the
     // end of the kernel before it (launch_pdl): 0.8 us between two kernels instead of 2.1, and no rounding up to ticks of 1 or 2 us,
     // which is how other launches of a stream start (e4m3 4 x 1024 12.3 -> 10.0 us a call, 32 x 4096 26.3 -> 23.9).

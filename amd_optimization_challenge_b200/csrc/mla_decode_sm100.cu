@@ -65,6 +65,7 @@ struct Misc {
     uint32_t tmem_base;
     int abort_flag;
     int meet;                             // outcome of the CTAs' meeting (MEET_*)
+    int q_share;                          // share of Q that this CTA looks at for another one, -1: all have been looked at
     int span[4];                          // first sequence, its first global tile, first and end tile of this CTA
     unsigned int q_red[8];                // cross-warp maximum of a split Q
     long long q_off[4];                   // element offset of each 16-row chunk of this row group inside a sequence's Q
@@ -272,6 +273,87 @@ __device__ __forceinline__ void find_span(const MlaParams& p, int w, int G, int 
     }
 }
 
+// largest magnitude of eight bf16 values, as its bit pattern (they order like their bit patterns)
+__device__ __forceinline__ unsigned int bf16x8_amax_bits(const uint4& v) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    unsigned int m = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) m = max(m, max(w[k] & 0x7fffu, (w[k] >> 16) & 0x7fffu));
+    return m;
+}
+// Maximum of Q that the CTAs find together, as a bit pattern.
+__device__ __forceinline__ unsigned int amax_bits(const int* status) { return *reinterpret_cast<const volatile unsigned int*>(status + SYNC_AMAX); }
+// One thread: a share of Q that is not marked in SYNC_AMAX_DONE, another one for each CTA as far as there are that many; -1 if there is
+// none, and then the other CTAs need not look either.
+__device__ __forceinline__ int open_share(int* status, int n_cta, int cta) {
+    auto open = [&](int i) {
+        const unsigned int all = n_cta - 32 * i >= 32 ? ~0u : (1u << (n_cta - 32 * i)) - 1u;
+        return ~(unsigned int)load_acquire(status + SYNC_AMAX_DONE + i) & all;
+    };
+    for (;;) {
+        int n = 0;
+#pragma unroll 1
+        for (int i = 0; 32 * i < n_cta; ++i) n += __popc(open(i));
+        if (n == 0) break;
+        int k = cta % n;
+#pragma unroll 1
+        for (int i = 0; 32 * i < n_cta; ++i) {
+            unsigned int o = open(i);
+            const int here = __popc(o);
+            if (k < here) {
+                for (; k > 0; --k) o &= o - 1;
+                return 32 * i + __ffs(o) - 1;
+            }
+            k -= here;
+        }                                                         // marked in between, at least one each time: look again
+    }
+    atomicOr(status + SYNC_AMAX_COUNT, 0x8000);
+    return -1;
+}
+// The softmax warps (SW of them, the first of the CTA) look at share c of a dense bf16 Q of `rows` rows: its maximum goes to SYNC_AMAX,
+// then its bit to SYNC_AMAX_DONE.  Twice does no harm.
+template <int SW>
+__device__ __forceinline__ void look_at_share(const uint4* q8, int rows, int* status, unsigned int n_cta, unsigned int c, unsigned int* q_red) {
+    constexpr int ST = 32 * SW, BATCH = 8;                        // loads in flight per thread
+    const unsigned long long n8 = (unsigned long long)rows * (QK_DIM / 8), end = n8 * (c + 1) / n_cta;
+    unsigned int m = 0;
+#pragma unroll 1
+    for (unsigned long long i = n8 * c / n_cta + threadIdx.x; i < end; i += BATCH * ST) {
+        uint4 v[BATCH];
+#pragma unroll
+        for (int k = 0; k < BATCH; ++k) v[k] = i + k * ST < end ? __ldcg(q8 + i + k * ST) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int k = 0; k < BATCH; ++k) m = max(m, bf16x8_amax_bits(v[k]));
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) q_red[threadIdx.x >> 5] = m;
+    named_bar_sync(3, ST);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < SW; ++k) m = max(m, q_red[k]);
+        atomicMax(reinterpret_cast<unsigned int*>(status + SYNC_AMAX), m);
+        __threadfence();
+        atomicOr(status + SYNC_AMAX_DONE + (c >> 5), 1 << (c & 31));
+    }
+}
+// Not all CTAs run yet: those that do look at the shares of the others, each at one that is open, until none is.  The maximum is in
+// q_red[0] then.  (When each looked at all of Q: 128 sequences of 128 heads, hybrid cache, limit 0, 1580 us a call; 362 so, 347 where all wait.)
+// Not inlined: registers of calls that never come here.
+template <int SW>
+__device__ __noinline__ void look_at_open_shares(const uint4* q8, int rows, int* status, int n_cta, int cta, unsigned int* q_red, int* q_share) {
+    for (;;) {
+        named_bar_sync(3, 32 * SW);                               // q_red has been read
+        if (threadIdx.x == 0) {
+            const int share = open_share(status, n_cta, cta);
+            *q_share = share;
+            if (share < 0) q_red[0] = amax_bits(status);
+        }
+        named_bar_sync(3, 32 * SW);
+        if (*q_share < 0) break;
+        look_at_share<SW>(q8, rows, status, n_cta, *q_share, q_red);
+    }
+}
+
 // Meeting of the CTAs (end of the kernel).  One thread: the CTAs that have come, every one that had when this began among them, and
 // their partials are visible.  A CTA sets its bit NO_BIT_CYCLES after being counted; the wait is bounded like mbar_wait.
 __device__ __forceinline__ void who_came(int* status, int n_cta, int (&mask)[UNIT_TOK], volatile int* abort_flag) {
@@ -369,14 +451,6 @@ __device__ __forceinline__ float fold_columns(const float (&x)[NC], int lane) {
     return v[0];
 }
 
-// largest magnitude of eight bf16 values, as its bit pattern (they order like their bit patterns)
-__device__ __forceinline__ unsigned int bf16x8_amax_bits(const uint4& v) {
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-    unsigned int m = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) m = max(m, max(w[k] & 0x7fffu, (w[k] >> 16) & 0x7fffu));
-    return m;
-}
 __device__ __forceinline__ f32x2 bf16x2_to_f32x2(uint32_t w) { return pk2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
 // eight bf16 values -> the eight e4m3 codes of q_cast_e4m3x8 (mla_common.cuh) in half the instructions: s2 = -scale and
 // r2 = RN(1 / scale), twice.  For values below general_from(r), which those of a tensor are of its own scale; a -0 may come out
@@ -485,28 +559,8 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
         const unsigned int lo = (w * per > 256u ? w * per - 256u : 0u) & ~31u, hi = min((w + 1) * per + 256u, n_ids);
         for (unsigned int i = lo + (tid - 32 * (SW + 2)) * 32; i < hi; i += 64 * 32) prefetch_l2(p.kv_indices + i);
     } else if (warp < SW && own_amax) {
-        constexpr int ST = 32 * SW, BATCH = 8;                    // loads in flight per thread
-        const unsigned int n_cta = gridDim.x * gridDim.y, c = blockIdx.y * gridDim.x + blockIdx.x;
-        const unsigned long long n8 = (unsigned long long)p.batch * p.rows * 72, end = n8 * (c + 1) / n_cta;
-        const uint4* q8 = reinterpret_cast<const uint4*>(p.q);
-        unsigned int m = 0;
-#pragma unroll 1
-        for (unsigned long long i = n8 * c / n_cta + tid; i < end; i += BATCH * ST) {
-            uint4 v[BATCH];
-#pragma unroll
-            for (int k = 0; k < BATCH; ++k) v[k] = i + k * ST < end ? __ldcg(q8 + i + k * ST) : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-            for (int k = 0; k < BATCH; ++k) m = max(m, bf16x8_amax_bits(v[k]));
-        }
-        m = __reduce_max_sync(0xffffffffu, m);
-        if (lane == 0) ms.q_red[warp] = m;
-        named_bar_sync(3, ST);
-        if (tid == 0) {
-#pragma unroll
-            for (int k = 0; k < SW; ++k) m = max(m, ms.q_red[k]);
-            atomicMax(reinterpret_cast<unsigned int*>(p.status + SYNC_AMAX), m);
-            red_release(p.status + SYNC_AMAX_COUNT, 1);
-        }
+        look_at_share<SW>(reinterpret_cast<const uint4*>(p.q), p.batch * p.rows, p.status, gridDim.x * gridDim.y, blockIdx.y * gridDim.x + blockIdx.x, ms.q_red);
+        if (tid == 0) atomicAdd(p.status + SYNC_AMAX_COUNT, 1);   // behind the fence of look_at_share
     }
     tc_fence_before();
     __syncthreads();
@@ -586,22 +640,15 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
                             }
                         } else {
                             if (q_scale_due) {                    // first use of the scale all CTAs contribute to: by now it is there
+                                const int n_cta = (int)(gridDim.x * gridDim.y);
                                 if (tid == 0)
-                                    ms.q_red[0] = count_reached(p.status + SYNC_AMAX_COUNT, (int)(gridDim.x * gridDim.y), p.meet_cycles)
-                                                      ? *reinterpret_cast<volatile unsigned int*>(p.status + SYNC_AMAX) : 0xffffffffu;
+                                    ms.q_red[0] = count_reached(p.status + SYNC_AMAX_COUNT, n_cta, p.meet_cycles) ? amax_bits(p.status) : 0xffffffffu;
                                 named_bar_sync(3, ST);
                                 unsigned int m = ms.q_red[0];
-                                if (m == 0xffffffffu) {           // not all CTAs run yet: this one looks at all of Q itself
-                                    const uint4* q8 = reinterpret_cast<const uint4*>(p.q);
-                                    m = 0;
-#pragma unroll 2
-                                    for (unsigned long long i = tid; i < (unsigned long long)p.batch * p.rows * 72; i += ST) m = max(m, bf16x8_amax_bits(__ldcg(q8 + i)));
-                                    m = __reduce_max_sync(0xffffffffu, m);
-                                    named_bar_sync(3, ST);        // q_red[0] has been read
-                                    if (lane == 0) ms.q_red[warp] = m;
-                                    named_bar_sync(3, ST);
-#pragma unroll
-                                    for (int k = 0; k < SW; ++k) m = max(m, ms.q_red[k]);
+                                if (__builtin_expect(m == 0xffffffffu, 0)) {
+                                    look_at_open_shares<SW>(reinterpret_cast<const uint4*>(p.q), p.batch * p.rows, p.status, n_cta,
+                                                            (int)(blockIdx.y * gridDim.x + blockIdx.x), ms.q_red, &ms.q_share);
+                                    m = ms.q_red[0];
 #pragma unroll
                                     for (int u = 0; u < 9; ++u) raw[u] = __ldcg(src + 8 * u);     // again: not kept over the loop
                                 }
@@ -1314,6 +1361,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
         if (tid == 0 && exited == n_cta - 1) {                    // the last one past the meeting: nobody looks at these any more
             p.status[SYNC_AMAX] = 0; p.status[SYNC_AMAX_COUNT] = 0; p.status[SYNC_PREFIX] = 0; p.status[SYNC_ARRIVE] = 0; p.status[SYNC_EXIT] = 0;
             for (int i = 0; i < SYNC_MASK_WORDS; i += 4) {
+                *reinterpret_cast<int4*>(p.status + SYNC_AMAX_DONE + i) = make_int4(0, 0, 0, 0);
                 *reinterpret_cast<int4*>(p.status + SYNC_ARRIVED + i) = make_int4(0, 0, 0, 0);
                 *reinterpret_cast<int4*>(p.status + SYNC_LEFT + i) = make_int4(0, 0, 0, 0);
             }

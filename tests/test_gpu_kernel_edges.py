@@ -157,10 +157,11 @@ def test_ctas_that_leave_before_the_merge(pkg, monkeypatch, kv_format, q_format,
     assert torch.equal(_run_over_nans(pkg, data, kv_format, q_format, impl="tcgen05", check_status=True), want)
 
 
-# What CTAs leave behind must not all fall on one of them: these calls took ten times as long then.
-@pytest.mark.parametrize("kv_format,q_format", [("fp8", "bf16")])
-def test_a_call_whose_ctas_leave_takes_little_longer(pkg, monkeypatch, kv_format, q_format):
-    data = pkg.generate_input(24, 1, 3000, seed=3, kv_lens=[3000] * 24, num_heads=128, formats=(kv_format,))
+# What CTAs leave behind must not all fall on one of them, and no CTA has to look at all of a large Q: these calls took ten times as
+# long when they did.
+@pytest.mark.parametrize("kv_format,q_format,lens", [("fp8", "bf16", [3000] * 24), ("fp8", "fp8", [100] * 600)])
+def test_a_call_whose_ctas_leave_takes_little_longer(pkg, monkeypatch, kv_format, q_format, lens):
+    data = pkg.generate_input(len(lens), 1, max(lens), seed=3, kv_lens=lens, num_heads=128, formats=(kv_format,))
 
     def us(n=20):
         times = []
