@@ -516,11 +516,9 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
     // Q quantised by this launch: its CTAs find the largest magnitude together, each in its share of Q
     const bool own_amax = !C::QSPLIT && p.q_cast && p.q_amax_parts == nullptr;
 
-    // Nothing of this touches memory that the kernel before may still write: it runs while that one drains.
-    if (warp == C::QK_WARP) {
-        tmem_alloc(&ms.tmem_base, C::TMEM_COLS);
-        tmem_relinquish();
-    } else if (tid == 32 * SW) {
+    // Nothing of this touches memory that the kernel before may still write: it runs while that one drains.  TMEM is taken later:
+    // a kernel before it that lets its dependents start early may not have its own columns yet, and would wait for this CTA, which waits for it.
+    if (tid == 32 * SW) {
         // a stage is full after one arrival per unit (copy loop, and the rope rows of a hybrid cache: also one per lane)
         for (int i = 0; i < NS; ++i) {
             mbar_init(&ms.kv_full[i], C::XF ? UNITS * (C::ROPE_SEP ? 33 : 1) : (use_tma ? UNITS : 32 * UNITS));
@@ -544,6 +542,10 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
     }
     __syncwarp();
     pdl_wait();
+    if (warp == C::QK_WARP) {
+        tmem_alloc(&ms.tmem_base, C::TMEM_COLS);
+        tmem_relinquish();
+    }
     if (warp == C::AUX_WARP) {
         int span[4];
         find_span<TILE>(p, w, G, lane, span, w == 0 && blockIdx.y == 0);
