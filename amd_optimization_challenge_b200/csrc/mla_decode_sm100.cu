@@ -1287,6 +1287,7 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
     };
     if (p.fused && warp >= SW) {
         looked_up = __shfl_sync(0xffffffffu, lane == 0 && load_acquire(p.status + SYNC_PREFIX) > 0, 0);
+        __syncwarp();                                             // lane 0 has acquired for all: a shuffle orders no memory accesses
         if (looked_up) look_up();
     }
     tc_fence_before();
