@@ -62,11 +62,17 @@ int sm_count() {
     return cached;
 }
 
-// MlaParams::meet_cycles: 50 us at 2 GHz, well above what the CTAs of a call are apart (they get equal shares; measured:
-// up to 10 us).  Testing aid: B200_MLA_MEET_CYCLES, 0 makes every CTA leave at once.
+// MlaParams::meet_cycles: 50 us at 2 GHz, well above what the CTAs of an ordinary call are apart (they get equal shares; measured:
+// up to 10 us).  Where shares are uneven by more, a CTA that goes costs the call nothing (see the merge in mla_decode_sm100.cu), so
+// the limit does not grow with the call.  Testing aid: B200_MLA_MEET_CYCLES, 0 makes a CTA go unless all have come when it first
+// looks; anything but a whole number from 0 to 2^30 is ignored.
 int meet_cycles() {
+    constexpr int usual = 100000;
     const char* e = getenv("B200_MLA_MEET_CYCLES");
-    return e && e[0] ? atoi(e) : 100000;
+    if (!e || e[0] < '0' || e[0] > '9') return usual;
+    char* end = nullptr;
+    const long long v = strtoll(e, &end, 10);
+    return *end == 0 && v <= 1 << 30 ? (int)v : usual;
 }
 
 constexpr int kMaxCtasPerSm = 2;

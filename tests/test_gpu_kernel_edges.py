@@ -157,6 +157,17 @@ def test_ctas_that_leave_before_the_merge(pkg, monkeypatch, kv_format, q_format,
     assert torch.equal(_run_over_nans(pkg, data, kv_format, q_format, impl="tcgen05", check_status=True), want)
 
 
+@pytest.mark.parametrize("text", ["", "soon", "-1", "0x", "0 us", "+0", " 0", "99999999999999999999"])
+def test_a_limit_that_is_no_number_is_ignored(pkg, monkeypatch, text):
+    data = pkg.generate_input(4, 1, 900, seed=4, kv_lens=[900] * 4)
+    _run(pkg, data, "fp8", "fp8", impl="tcgen05")
+    before = _left(pkg)
+    monkeypatch.setenv("B200_MLA_MEET_CYCLES", text)
+    for _ in range(5):
+        _run(pkg, data, "fp8", "fp8", impl="tcgen05")
+    assert _left(pkg) == before
+
+
 # What CTAs leave behind must not all fall on one of them, and no CTA has to look at all of a large Q: these calls took ten times as
 # long when they did.
 @pytest.mark.parametrize("kv_format,q_format,lens", [("fp8", "bf16", [3000] * 24), ("fp8", "fp8", [100] * 600)])
