@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from helpers import assert_close, oracle_for_data
+from oracle import mla_oracle as mo
 
 pytestmark = pytest.mark.gpu
 
@@ -221,6 +222,90 @@ def test_decode_behind_other_work_of_the_stream(pkg, kv_format, q_format):
         assert all(torch.equal(o, want[i & 1]) for i, o in enumerate(outs))
 
 
+def _eager_and_captured(steps, want, rounds=3):
+    """Every step's output, eagerly one after the other and as a graph."""
+    outs = [step() for _ in range(rounds) for step in steps]
+    for i, o in enumerate(outs):
+        assert torch.equal(o, want[i % len(want)]), i
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        outs = [step() for step in steps]
+    for _ in range(rounds):
+        graph.replay()
+        torch.cuda.synchronize()
+        for i, o in enumerate(outs):
+            assert torch.equal(o, want[i]), i
+
+
+# Only the edge between two kernels is relaxed (a copy before the decode orders it fully): here a kernel has written each of the
+# inputs in turn just before the decode, with inputs that change from call to call.
+@pytest.mark.parametrize("kv_format,q_format", [("fp8", "fp8"), ("fp8", "bf16"), ("mxfp4", "bf16"), ("hybrid", "fp8")])
+def test_decode_behind_the_kernel_that_wrote_an_input(pkg, kv_format, q_format):
+    lens = ([3000, 17, 900, 64], [64, 900, 17, 3000])
+    sets = [pkg.generate_input(4, 1, 3000, seed=s, kv_lens=l, shuffle_pages=True, formats=(kv_format,)) for s, l in zip((1, 2), lens)]
+    want = [_run(pkg, d, kv_format, q_format) for d in sets]
+    assert not torch.equal(*want)
+    inputs = [(d[0], d[3], d[4]["kv_indices"], *d[1][kv_format]) for d in sets]
+    own = [t.clone() for t in inputs[0]]
+    data = (own[0], {kv_format: tuple(own[3:])}, sets[0][2], own[1], dict(sets[0][4], kv_indices=own[2]))
+
+    def write(to, new):
+        if to.dtype in (torch.bfloat16, torch.float32):
+            torch.maximum(new, new, out=to)
+        else:                                                    # indices, and bytes of every kind
+            kind = torch.int32 if to.dtype is torch.int32 else torch.uint8
+            torch.bitwise_or(new.view(kind), new.view(kind), out=to.view(kind))
+
+    def step(i, last):
+        order = [k for k in range(len(own)) if k != last] + [last]
+        for k in order:
+            write(own[k], inputs[i][k])
+        return _run(pkg, data, kv_format, q_format)
+
+    todo = [(n & 1, n % len(own)) for n in range(2 * len(own))] + [(n + 1 & 1, n % len(own)) for n in range(2 * len(own))]
+    torch.cuda.synchronize()
+    _eager_and_captured([lambda i=i, last=last: step(i, last) for i, last in todo], [want[i] for i, _ in todo])
+
+
+# The same behind the library's own kernels: rows appended, Q quantised, and partials that a merge still reads.
+@pytest.mark.parametrize("kv_format", ["fp8", "mxfp4", "hybrid"])
+def test_decode_behind_kernels_of_the_library(pkg, kv_format):
+    lens = [3000, 17, 900, 64]
+    n, heads = sum(lens), 16
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rows = [torch.randn(n, 576, generator=g, device="cuda").bfloat16() for _ in range(2)]
+    qs = [torch.randn(4, heads, 576, generator=g, device="cuda").bfloat16() for _ in range(2)]
+    slots = torch.randperm(n, generator=g, device="cuda").to(torch.int32)
+    planes = {"fp8": pkg.quantize_fp8, "mxfp4": pkg.quantize_mxfp4, "hybrid": pkg.quantize_hybrid}[kv_format](rows[0][:, None])
+    planes = tuple(t.clone() for t in planes)
+    ip = torch.tensor([0, 3000, 3017, 3917, 3981], dtype=torch.int32, device="cuda")
+    n_o = 4 * heads * 512
+    record = torch.empty(2 * (n_o + 4 * heads), device="cuda")
+    parts = [(r[:n_o].view(4, heads, 512), r[n_o:].view(4, heads)) for r in record.chunk(2)]
+
+    def step(i, last, wait):
+        pause = torch.cuda.synchronize if wait else lambda: None
+        if last == "append":
+            q, scale = pkg.quantize_q_fp8(qs[i])
+            pause()
+        pkg.kv_append(rows[i], kv_format, planes, slots=slots)
+        pause()
+        if last == "quantise":
+            q, scale = pkg.quantize_q_fp8(qs[i])
+            pause()
+        for part in parts:
+            pkg.mla_decode(q, scale, kv_format, planes, ip, sm_scale=0.05, kv_indices=slots, return_partial=True, partial_out=part)
+            pause()
+        out = pkg.submission.combine_partials_strided(record, 2, record.numel() // 2, n_o, 4, heads)
+        pause()
+        return out
+
+    todo = [(k & 1, last) for k in range(4) for last in ("append", "quantise")] + [(k + 1 & 1, last) for k in range(4) for last in ("quantise", "append")]
+    want = [step(i, last, True) for i, last in todo]
+    assert not torch.equal(want[0], want[2])
+    _eager_and_captured([lambda i=i, last=last: step(i, last, False) for i, last in todo], want)
+
+
 # The span search gives a lane ceil(batch / 32) sequences and looks inside them 32 at a time.
 @pytest.mark.parametrize("batch", [31, 32, 33, 64, 65, 300, 1025])
 def test_batches_around_the_lanes_of_the_span_search(pkg, batch):
@@ -335,7 +420,8 @@ def test_coherent_tail_far_below_the_maximum(pkg, heads, depth, at):
 
 
 # Scores that climb along the sequence, for different rows at different tiles, so that reference maxima move and O is rescaled
-# again and again.  Against the warp-level kernel; bf16 outputs and probabilities of about eight bits on either side.
+# again and again.  Against the fp32 oracle: a bf16 output (2^-9), probabilities of about eight bits (2^-9), Q and cache as they are
+# stored; with as much again for their sum.
 @pytest.mark.parametrize("kv_format,q_format,heads", [("fp8", "fp8", 16), ("fp8", "bf16", 32), ("fp8", "fp8", 64), ("fp8", "fp8", 128),
                                                       ("mxfp4", "bf16", 16), ("mxfp4", "bf16", 32), ("mxfp4", "fp8", 64), ("hybrid", "fp8", 128)])
 def test_reference_maxima_that_move_at_most_tiles(pkg, kv_format, q_format, heads):
@@ -352,10 +438,11 @@ def test_reference_maxima_that_move_at_most_tiles(pkg, kv_format, q_format, head
     planes, q = quantise(kv.bfloat16().cuda()), q.bfloat16().cuda()
     qc, qs = pkg.quantize_q_fp8(q) if q_format == "fp8" else (q, None)
     ip = torch.tensor([0, 1500, 1597, 2297], dtype=torch.int32, device="cuda")
-    run = lambda **kw: pkg.mla_decode(qc, qs, kv_format, planes, ip, sm_scale=1.0, **kw).float()
-    want = run(impl="generic")
-    for max_ctas in (1, 0):                                      # one CTA per row group, and spread out
-        got = run(impl="tcgen05", max_ctas=max_ctas)
+    run = lambda **kw: pkg.mla_decode(qc, qs, kv_format, planes, ip, sm_scale=1.0, **kw).float().cpu()
+    want = mo.decode_from_data(qc.cpu(), None if qs is None else qs.cpu(), kv_format, tuple(t.cpu() for t in planes), ip.cpu().numpy(), None,
+                               1.0).float()
+    for kw in (dict(impl="generic"), dict(impl="tcgen05", max_ctas=1), dict(impl="tcgen05")):      # one CTA per row group, and spread out
+        got = run(**kw).reshape(want.shape)
         assert torch.isfinite(got).all()
         assert float((got - want).norm() / want.norm()) <= 2.0 ** -7
 
