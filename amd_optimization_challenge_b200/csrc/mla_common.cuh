@@ -148,11 +148,9 @@ __device__ __forceinline__ void store_bf16x4(__nv_bfloat16* dst, float4 v) {
     *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<uint2*>(o);
 }
 
-// Where partials are and merged rows go (see MlaParams).
-struct MergeIo { const float *part_o, *part_lse; __nv_bfloat16* out; float *out_o_f32, *out_lse; int rows; };
 
-template <int V, int U, typename Io>
-__device__ __forceinline__ void merge_row(const Io& p, int b, int r, int w0, int w1, int d) {
+template <int V, int U>
+__device__ __forceinline__ void merge_row(const MlaParams& p, int b, int r, int w0, int w1, int d) {
     const long long orow = (long long)b * p.rows + r;
     float M = -INFINITY, den = 0.f;
     float4 acc[V];

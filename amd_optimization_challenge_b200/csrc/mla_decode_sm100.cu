@@ -332,7 +332,7 @@ __device__ __forceinline__ void look_at_share(const uint4* q8, int rows, int* st
 #pragma unroll
         for (int k = 0; k < SW; ++k) m = max(m, q_red[k]);
         atomicMax(reinterpret_cast<unsigned int*>(status + SYNC_AMAX), m);
-        __threadfence();
+        fence_acq_rel();
         atomicOr(status + SYNC_AMAX_DONE + (c >> 5), 1 << (c & 31));
     }
 }
@@ -397,16 +397,68 @@ __device__ __forceinline__ int next_shared(const MlaParams& p, int b0, int w, in
 }
 
 // One item of the merge: row r of sequence b (sh = 0), a half (1) or a quarter of it (2), which `item` tells.
-template <typename Io>
-__device__ __forceinline__ void merge_item(const Io& io, int b, int r, int w0, int w1, int item, int sh, int lane) {
-    if (sh == 2) merge_row<1, 12>(io, b, r, w0, w1, (item & 3) * 128 + lane * 4);
-    else if (sh == 1) merge_row<2, 6>(io, b, r, w0, w1, (item & 1) * 256 + lane * 4);
-    else merge_row<4, 4>(io, b, r, w0, w1, lane * 4);
+__device__ __forceinline__ void merge_item(const MlaParams& p, int b, int r, int w0, int w1, int item, int sh, int lane) {
+    if (sh == 2) merge_row<1, 12>(p, b, r, w0, w1, (item & 3) * 128 + lane * 4);
+    else if (sh == 1) merge_row<2, 6>(p, b, r, w0, w1, (item & 1) * 256 + lane * 4);
+    else merge_row<4, 4>(p, b, r, w0, w1, lane * 4);
 }
-// The same code for CTAs that did not all come in time.  Not inlined: a second copy inside the kernel cost the calls that never reach
-// it registers (4-byte spills; e4m3 32 x 4096 24.15 us, 23.9 so).
-__device__ __noinline__ void merge_item_late(MergeIo io, int b, int r, int w0, int w1, int item, int sh, int lane) {
-    merge_item(io, b, r, w0, w1, item, sh, lane);
+// Not all CTAs have come in NO_BIT_CYCLES, or some had left when this one came (`seen`: SYNC_ARRIVE before it was counted).  One thread; returns
+// the outcome of the meeting.  This and merge_late are not inlined: inside the kernel they cost the calls that never reach them
+// registers (4-byte spills; e4m3 32 x 4096 24.15 us, 23.9 so).
+__device__ __noinline__ int meet_late(Misc& ms, int* status, int n_cta, int cta, int seen, bool all, int cycles) {
+    int* arrive = status + SYNC_ARRIVE;
+    const int bit = 1 << (cta & 31);
+    int meet = 0;
+    or_release(status + SYNC_ARRIVED + (cta >> 5), bit);
+    if (seen >> 16) {
+        meet = MEET_LATE;
+        who_came(status, n_cta, ms.mask(MASK_LATE_ARRIVED), &ms.abort_flag);
+        for (int i = 0; i < SYNC_MASK_WORDS; ++i) ms.mask(MASK_LATE_LEFT)[i] = load_acquire(status + SYNC_LEFT + i);
+    }
+    if (!all) all = count_reached(arrive, n_cta, cycles);
+    if (!all) {
+        atomicOr(status + SYNC_LEFT + (cta >> 5), bit);
+        all = (add_acq_rel(arrive, 1 << 16) & 0xffff) == n_cta;
+    }
+    if (!all) {
+        meet |= MEET_LEFT;
+        who_came(status, n_cta, ms.mask(MASK_ARRIVED), &ms.abort_flag);
+        atomicAdd(status + ST_LEAVES, 1);
+    }
+    if (meet && load_acquire(status + SYNC_PREFIX) == 0) meet |= MEET_NO_TABLE;
+    return meet;
+}
+// The merge by a CTA that has left before the last came, or come after others had left.  All its threads; N rows per CTA.
+template <int TILE, int N>
+__device__ __noinline__ void merge_late(const MlaParams& p, Misc& ms, int first_item, int sh) {
+    const int meet = ms.meet, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int w = blockIdx.x, y0 = blockIdx.y, G = gridDim.x, n_cta = G * gridDim.y;
+    if (meet & MEET_NO_TABLE) {                                   // the first CTA has not begun: the same table, by this one
+        if (warp == 0) {
+            int s0, s1, mine;
+            const int incl = lane_tiles<TILE>(p, lane, s0, s1, mine);
+            write_seq_ctas<TILE>(p, make_sched(__shfl_sync(0xffffffffu, incl, 31), p.batch, G, p.seq_units), s0, s1, incl - mine);
+        }
+        __syncthreads();
+    }
+    int item = first_item, end = p.batch * p.rows << sh, heir_of = -1;       // >= 0: rows that others have left of this sequence
+    for (;;) {
+        for (; item < end; item += heir_of < 0 ? n_cta * warps : warps) {
+            const int b = (item >> sh) / p.rows, r = (item >> sh) - b * p.rows, y = r / N;
+            const int2 ctas = __ldcg(p.seq_ctas + b);
+            if (ctas.x != ctas.y && (heir_of >= 0 ? in_mask(ms.mask(MASK_LATE_LEFT), item % n_cta, item % n_cta)
+                                                  : !(meet & MEET_LEFT) || in_mask(ms.mask(MASK_ARRIVED), y * G + ctas.x, y * G + ctas.y)))
+                merge_item(p, b, r, ctas.x, ctas.y, item, sh, lane);
+        }
+        if (!(meet & MEET_LATE)) break;
+        int2 ctas;                                                // the next sequence that this CTA shares with others
+        if (heir_of < 0) heir_of = ms.span[0] - 1;
+        do heir_of = next_shared(p, heir_of + 1, w, lane, ctas);
+        while (heir_of < p.batch && !in_mask(ms.mask(MASK_LATE_ARRIVED), y0 * G + ctas.x, y0 * G + ctas.y));
+        if (heir_of >= p.batch) break;
+        end = (heir_of * p.rows + (y0 + 1) * N) << sh;
+        item = ((heir_of * p.rows + y0 * N) << sh) + warp;
+    }
 }
 
 // Position of one role inside the CTA's span: the sequence of the current tile and its geometry.
@@ -501,7 +553,7 @@ __device__ __forceinline__ uint32_t operand_offset(int r, int c) {
 
 template <int N, int KVFMT, int QFMT>
 __global__ void __launch_bounds__(Cfg<N, KVFMT, QFMT>::THREADS, 1)
-mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, const bool use_tma) {
+mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_constant__ Maps maps, const bool use_tma) {
     using C = Cfg<N, KVFMT, QFMT>;
     constexpr int NQ = C::NQ, NC = C::NC, SW = C::SW, FW = C::FW, TILE = C::TILE, NS = C::NS, UNITS = C::UNITS;
     constexpr int PANEL_BYTES = C::PANEL_BYTES, STAGE_BYTES = C::STAGE_BYTES, P_BUFS = C::P_BUFS;
@@ -542,10 +594,6 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
     }
     __syncwarp();
     pdl_wait();
-    if (warp == C::QK_WARP) {
-        tmem_alloc(&ms.tmem_base, C::TMEM_COLS);
-        tmem_relinquish();
-    }
     if (warp == C::AUX_WARP) {
         int span[4];
         find_span<TILE>(p, w, G, lane, span, w == 0 && blockIdx.y == 0);
@@ -563,6 +611,10 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
     } else if (warp < SW && own_amax) {
         look_at_share<SW>(reinterpret_cast<const uint4*>(p.q), p.batch * p.rows, p.status, gridDim.x * gridDim.y, blockIdx.y * gridDim.x + blockIdx.x, ms.q_red);
         if (tid == 0) atomicAdd(p.status + SYNC_AMAX_COUNT, 1);   // behind the fence of look_at_share
+    }
+    if (warp == C::QK_WARP) {
+        tmem_alloc(&ms.tmem_base, C::TMEM_COLS);
+        tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
@@ -1296,70 +1348,19 @@ mla_decode_sm100_kernel(const MlaParams p, const __grid_constant__ Maps maps, co
     if (p.fused) {
         int exited = 0;
         if (tid == 0) {                                           // after the __syncthreads: covers the stores of the whole CTA
-            int* arrive = p.status + SYNC_ARRIVE;
-            const int bit = 1 << (cta & 31);
-            const int seen = add_acq_rel(arrive, 1);
+            const int seen = add_acq_rel(p.status + SYNC_ARRIVE, 1);
             bool all = (seen & 0xffff) == n_cta - 1;
-            int meet = 0;
-            if (!all && !(seen >> 16)) all = count_reached(arrive, n_cta, min(p.meet_cycles, NO_BIT_CYCLES));
-            if (__builtin_expect(!all || seen >> 16, 0)) {
-                or_release(p.status + SYNC_ARRIVED + (cta >> 5), bit);
-                if (seen >> 16) {
-                    meet = MEET_LATE;
-                    who_came(p.status, n_cta, ms.mask(MASK_LATE_ARRIVED), abort_flag);
-                    for (int i = 0; i < SYNC_MASK_WORDS; ++i) ms.mask(MASK_LATE_LEFT)[i] = load_acquire(p.status + SYNC_LEFT + i);
-                }
-                if (!all) all = count_reached(arrive, n_cta, p.meet_cycles);
-                if (!all) {
-                    atomicOr(p.status + SYNC_LEFT + (cta >> 5), bit);
-                    all = (add_acq_rel(arrive, 1 << 16) & 0xffff) == n_cta;
-                }
-                if (!all) {
-                    meet |= MEET_LEFT;
-                    who_came(p.status, n_cta, ms.mask(MASK_ARRIVED), abort_flag);
-                    atomicAdd(p.status + ST_LEAVES, 1);
-                }
-                if (meet && load_acquire(p.status + SYNC_PREFIX) == 0) meet |= MEET_NO_TABLE;
-            }
-            ms.meet = meet;
+            if (!all && !(seen >> 16)) all = count_reached(p.status + SYNC_ARRIVE, n_cta, min(p.meet_cycles, NO_BIT_CYCLES));
+            ms.meet = __builtin_expect(all && !(seen >> 16), 1) ? 0 : meet_late(ms, p.status, n_cta, cta, seen, all, p.meet_cycles);
         }
         __syncthreads();
         if (tid == 0) exited = atomicAdd(p.status + SYNC_EXIT, 1);        // looked at after the merge
-        const int meet = ms.meet;
-        if (__builtin_expect(meet == 0, 1)) {
+        if (__builtin_expect(ms.meet == 0, 1)) {
             if (!looked_up) look_up();
             for (; (item >> sh) < rows_all; item += n_warps, look_up())
                 if (work) merge_item(p, b, (item >> sh) - b * p.rows, w0, w1, item, sh, lane);
         } else {
-            if (meet & MEET_NO_TABLE) {                           // the first CTA has not begun: the same table, by this one
-                if (warp == 0) {
-                    int s0, s1, mine;
-                    const int incl = lane_tiles<TILE>(p, lane, s0, s1, mine);
-                    write_seq_ctas<TILE>(p, make_sched(__shfl_sync(0xffffffffu, incl, 31), p.batch, G, p.seq_units), s0, s1, incl - mine);
-                }
-                __syncthreads();
-            }
-            look_up();
-            int end = rows_all << sh, heir_of = -1;               // >= 0: rows that others have left of this sequence
-            for (;;) {
-                for (; item < end; item += heir_of < 0 ? n_warps : WARPS, look_up()) {
-                    if (!work) continue;
-                    const int r = (item >> sh) - b * p.rows, y = r / N;
-                    if (heir_of >= 0 ? in_mask(ms.mask(MASK_LATE_LEFT), item % n_cta, item % n_cta)
-                                     : !(meet & MEET_LEFT) || in_mask(ms.mask(MASK_ARRIVED), y * G + w0, y * G + w1))
-                        merge_item_late(MergeIo{p.part_o, p.part_lse, p.out, p.out_o_f32, p.out_lse, p.rows}, b, r, w0, w1, item, sh, lane);
-                }
-                if (!(meet & MEET_LATE)) break;
-                int2 ctas;                                        // the next sequence that this CTA shares with others
-                if (heir_of < 0) heir_of = ms.span[0] - 1;
-                do heir_of = next_shared(p, heir_of + 1, (int)blockIdx.x, lane, ctas);
-                while (heir_of < p.batch && !in_mask(ms.mask(MASK_LATE_ARRIVED), blockIdx.y * G + ctas.x, blockIdx.y * G + ctas.y));
-                if (heir_of >= p.batch) break;
-                item = heir_of * p.rows + (int)blockIdx.y * N;
-                end = (item + N) << sh;
-                item = (item << sh) + warp;
-                look_up();
-            }
+            merge_late<TILE, N>(p, ms, item, sh);
         }
         if (tid == 0 && exited == n_cta - 1) {                    // the last one past the meeting: nobody looks at these any more
             p.status[SYNC_AMAX] = 0; p.status[SYNC_AMAX_COUNT] = 0; p.status[SYNC_PREFIX] = 0; p.status[SYNC_ARRIVE] = 0; p.status[SYNC_EXIT] = 0;

@@ -90,6 +90,7 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, const uint4& v) {
 __device__ __forceinline__ void red_release(int* counter, int v) {
     asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(counter), "r"(v) : "memory");
 }
+__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 __device__ __forceinline__ void or_release(int* word, int bits) {
     asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(word), "r"(bits) : "memory");
 }
