@@ -119,5 +119,5 @@ def test_tmem_is_taken_behind_the_wait_for_the_kernel_before():
     """A decode CTA may run beside the kernel before it.  If it held TMEM columns while it waits for that kernel, and that one had
     yet to allocate its own, neither would go on.  Read from the source: such a run must not happen on a GPU."""
     src = open(os.path.join(ROOT, "amd_optimization_challenge_b200", "csrc", "mla_decode_sm100.cu")).read()
-    kernel = src[src.index("mla_decode_sm100_kernel(const MlaParams p"):]
+    kernel = src[src.index("mla_decode_sm100_kernel(const "):]
     assert 0 < kernel.index("pdl_wait();") < kernel.index("tmem_alloc(")
