@@ -368,7 +368,7 @@ __device__ __forceinline__ void who_came(int* status, int n_cta, int (&mask)[UNI
         }
         const int count = load_acquire(status + SYNC_ARRIVE) & 0xffff;
         if (bits == count) return;
-        if (count == n_cta) break;
+        if (count >= n_cta) break;
         if (*abort_flag || clock64() - t0 > WAIT_LIMIT_CYCLES) { *abort_flag = 1; break; }
     }
     for (int i = 0; i < SYNC_MASK_WORDS; ++i) mask[i] = -1;
