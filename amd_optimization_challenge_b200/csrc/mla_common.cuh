@@ -1,5 +1,5 @@
 // Shared device-side definitions for the MLA decode kernels: kernel parameter block, the
-// KV-span schedule that every CTA and the merge derive from kv_indptr, and the
+// KV-span schedule that every CTA derives from kv_indptr, the merge of partials, and the
 // byte-format decoders (e4m3fn, e2m1 + E8M0).
 #pragma once
 
@@ -25,9 +25,10 @@ enum { KV_E4M3 = 0, KV_MXFP4 = 1, KV_HYBRID = 2 };
 // Bits of the sticky status word at the head of the workspace (B200_MLA_STATUS_* in b200_mla.h).
 enum { ST_OK = 0, ST_TIMEOUT = 1, ST_BAD_PAGE = 2 };
 
-// Launch of a kernel whose first statement is pdl_wait(): its blocks are placed while the kernel before it in the stream
+// Launch of a kernel all of whose threads call pdl_wait(): its blocks are placed while the kernel before it in the stream
 // drains, which leaves 1 us between the two instead of 3 us.  pdl_wait returns when that kernel is complete and its writes
-// are visible, so nothing may be read or written before it.  What that kernel may have written is read with __ldcg or
+// are visible.  Before it a block may set up its own shared memory and nothing else: no global memory is read or written, and nothing
+// taken that the kernel before could wait for (TMEM columns).  All but the decode kernel call it first of all.  What that kernel may have written is read with __ldcg or
 // load_global: __ldg is for data that nobody writes while the kernel runs, and its blocks run already.
 template <typename... Params, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, unsigned int threads, unsigned int smem, cudaStream_t stream, const Args&... args) {
@@ -44,9 +45,9 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 
 // Words of the 256-byte workspace header behind the status word.  ST_FORWARD: address (two words) of a second status word that
 // receives the same bits, 0 if there is none.  ST_LEAVES: how many CTAs have left a meeting before all had come, in all launches
-// so far (for tests and measurements).  SYNC_*: for launches whose CTAs work together; they are zero between launches: the last
+// so far (for tests and measurements).  SYNC_TABLE: MlaParams::seq_ctas has been written.  SYNC_*: for launches whose CTAs work together; they are zero between launches: the last
 // CTA to exit resets them.  SYNC_AMAX_DONE, SYNC_ARRIVED, SYNC_LEFT: SYNC_MASK_WORDS words each, one bit per CTA.
-enum { ST_FORWARD = 2, ST_LEAVES = 4, SYNC_AMAX = 16, SYNC_AMAX_COUNT = 17, SYNC_PREFIX = 18, SYNC_AMAX_DONE = 20, SYNC_ARRIVE = 32, SYNC_ARRIVED = 36, SYNC_EXIT = 48,
+enum { ST_FORWARD = 2, ST_LEAVES = 4, SYNC_AMAX = 16, SYNC_AMAX_COUNT = 17, SYNC_TABLE = 18, SYNC_AMAX_DONE = 20, SYNC_ARRIVE = 32, SYNC_ARRIVED = 36, SYNC_EXIT = 48,
        SYNC_LEFT = 52, SYNC_MASK_WORDS = 8 };
 constexpr int MAX_FUSED_CTAS = 32 * SYNC_MASK_WORDS;
 

@@ -28,11 +28,12 @@
 //        1 QK warp, 1 PV warp (the whole warp runs the loop, one elected lane issues), for a block-scaled cache 2 fetch warps
 //        (the PV warp, or the first fetch warp, searches the CTA's span before that)
 // What bounds it, and microseconds a call before (a kernel per family, maximum of Q and merge as launches of their own, one
-// issuing warp) and now: e4m3 256 x 8192 the HBM rate (264 -> 198), 128 heads over an e4m3 cache the chain load -> QK -> softmax -> PV
-// of two stages (236 -> 79), MXFP4 64 x 8192 the same chain with the conversion in it (96 -> 63), MXFP4 8 x 131072 with two
-// queries and hybrid 128 heads shared memory, conversion and MMA operands alike (214 -> 141, 640 -> 382), e4m3 4 x 1024 latencies (23.5 -> 10.0).
+// issuing warp) and now: e4m3 256 x 8192 the HBM rate (264 -> 211), 128 heads over an e4m3 cache the chain load -> QK -> softmax -> PV
+// of two stages (236 -> 80), MXFP4 64 x 8192 the same chain with the conversion in it (96 -> 64), MXFP4 8 x 131072 with two
+// queries and hybrid 128 heads shared memory, conversion and MMA operands alike (214 -> 144, 640 -> 384), e4m3 4 x 1024 latencies
+// (23.5 -> 10.0 to 10.6).  Long calls vary by 8 % from GPU to GPU.
 // Synchronisation is mbarrier based; every such wait is bounded and on expiry sets a status word.  The two waits for other CTAs
-// are shorter and need no status: see MlaParams::meet_cycles.
+// are shorter, and who gives up goes on without them and sets no status: see MlaParams::meet_cycles.
 //
 // Role in the reference: the split-KV stage-1 kernels (mixed-mla/submission.py:122-250,
 // mixed-mla/versions/hip_mxfp4_v5/submission.py:214-656) and their block decode (mixed-mla/triton_mla_mxfp4.py:20-67).
@@ -102,7 +103,7 @@ struct Cfg {
     // A probability p (relative to the reference maximum) is stored as 2^P_SCALE_LOG2 p; a score more than RECENTER log2 units above
     // the reference maximum moves it.  2^(P_SCALE_LOG2 + RECENTER) must stay below 448.  The smallest step of the stored pair is
     // 2^-13 with lo / 16 in columns of its own, 2^-9 where lo shares hi's columns (MERGED): there the larger factor keeps the same
-    // 2^-17 below the reference maximum, at the price of moving it at most tiles (48 ragged sequences of 128 heads: 81 us; 85 when
+    // 2^-17 below the reference maximum, at the price of moving it at most tiles (48 ragged sequences of 128 heads: 80 us; 85 when
     // O was rescaled before the probabilities were computed, all of it, and the scores read three times; less with 2^4, but like
     // keys 12 binades down come out 28 % wrong).  Block-scaled caches at 64 rows keep 2^4, i.e. 2^-13.
     static constexpr bool DEEP = MERGED && !XF;
@@ -269,7 +270,7 @@ __device__ __forceinline__ void find_span(const MlaParams& p, int w, int G, int 
     span[0] = seq; span[1] = seq_t0; span[2] = t_first; span[3] = t_end;
     if (write_table) {
         write_seq_ctas<TILE>(p, sc, s0, s1, incl - mine);
-        if (lane == 0 && p.fused) red_release(p.status + SYNC_PREFIX, 1);      // cumulative: __syncwarp orders the lanes' stores before it
+        if (lane == 0 && p.fused) red_release(p.status + SYNC_TABLE, 1);      // cumulative: __syncwarp orders the lanes' stores before it
     }
 }
 
@@ -425,7 +426,7 @@ __device__ __noinline__ int meet_late(Misc& ms, int* status, int n_cta, int cta,
         who_came(status, n_cta, ms.mask(MASK_ARRIVED), &ms.abort_flag);
         atomicAdd(status + ST_LEAVES, 1);
     }
-    if (meet && load_acquire(status + SYNC_PREFIX) == 0) meet |= MEET_NO_TABLE;
+    if (meet && load_acquire(status + SYNC_TABLE) == 0) meet |= MEET_NO_TABLE;
     return meet;
 }
 // The merge by a CTA that has left before the last came, or come after others had left.  All its threads; N rows per CTA.
@@ -890,7 +891,9 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
                     }
                 };
                 // x = scores relative to the reference maxima (to zero at a sequence's first tile, see nm); from here on the
-                // tile lives in registers and the S buffer goes back
+                // tile lives in registers and the S buffer goes back.  Where a maximum moves, x is shifted: rounded twice, the first time at
+                // the size it had before, where one FMA with the new maximum rounds once.  That is half an ulp of a score, which the sum over
+                // 18 k-steps carries anyway: errors against 64 bits agree to three digits with those of the FMA up to scores of 158.
                 if (active) {
                     load_scores(ms.nm[sg][nm_cur]);
                     mask_scores();
@@ -1314,12 +1317,14 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
     // quarters: spills, 32.9 us for a rank of eight instead of 31.2).
     // The launch is not cooperative (see MlaParams::meet_cycles): a CTA that has waited meet_cycles for the others goes.  It says so (its
     // bit in SYNC_LEFT, then one in the upper half of SYNC_ARRIVE), looks who has come, and merges those rows of its share whose
-    // partials are all there.  A row that it has to leave behind lacks a CTA that comes later.  That one learns from SYNC_ARRIVE that
+    // partials are all there.  A row that it has to leave behind lacks a CTA that comes later; that one learns from SYNC_ARRIVE that
     // others had left, and the last CTA of a sequence to come merges what those have left of it.  So what falls on a late CTA is rows of the
-    // one or two sequences that it shares with others, in its row group: 64 rows of 74 partials at most, 10 MB.  When all of it fell on the last
-    // CTA of the call, 50 us of waiting in vain became several hundred of merging by one CTA (us a call: 500 sequences of 3 tokens, 500 of 700
-    // and 20 of 100000 in turn, 128 heads over an e4m3 cache, 1447, 872 so and 937 if every CTA waits for all; 3000 of 5 and 30 of 300000,
-    // MXFP4, 2315, 1115 and 1162; 48 sequences of 128 heads with a limit of 0, 753 and 90, where 78 is without anyone leaving).
+    // one or two sequences that it shares with others, in its row group: 64 rows of 74 partials at most, 10 MB and 270 us for one CTA (one
+    // sequence of 131072 tokens, 128 heads, one SM held by another stream: 450 us, 64 without that).
+    // When all of it fell on the last CTA of the call, 50 us of waiting in vain became several hundred of merging by one CTA (us a call: 500
+    // sequences of 3 tokens, 500 of 700 and 20 of 100000 mixed, 128 heads over an e4m3 cache, 1447, 865 so and 937 if every CTA waits for
+    // all; 3000 of 5 and 30 of 300000, MXFP4, 2315, 1127 and 1162; 48 sequences of 128 heads with a limit of 0, 753 and 90, where 78 is
+    // without anyone leaving).
     // Two that write a row (a CTA that learns only as it goes that all have come merges its share after all) write the same values.
     // Who has come is read from SYNC_ARRIVED, whose bits are set after the count: a look that shows as many bits as the count
     // read after it shows every CTA that had come by then.
@@ -1338,7 +1343,7 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
         work = w0 != w1;                                          // one CTA has finished the sequence; none: zeros
     };
     if (p.fused && warp >= SW) {
-        looked_up = __shfl_sync(0xffffffffu, lane == 0 && load_acquire(p.status + SYNC_PREFIX) > 0, 0);
+        looked_up = __shfl_sync(0xffffffffu, lane == 0 && load_acquire(p.status + SYNC_TABLE) > 0, 0);
         __syncwarp();                                             // lane 0 has acquired for all: a shuffle orders no memory accesses
         if (looked_up) look_up();
     }
@@ -1363,7 +1368,7 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
             merge_late<TILE, N>(p, ms, item, sh);
         }
         if (tid == 0 && exited == n_cta - 1) {                    // the last one past the meeting: nobody looks at these any more
-            p.status[SYNC_AMAX] = 0; p.status[SYNC_AMAX_COUNT] = 0; p.status[SYNC_PREFIX] = 0; p.status[SYNC_ARRIVE] = 0; p.status[SYNC_EXIT] = 0;
+            p.status[SYNC_AMAX] = 0; p.status[SYNC_AMAX_COUNT] = 0; p.status[SYNC_TABLE] = 0; p.status[SYNC_ARRIVE] = 0; p.status[SYNC_EXIT] = 0;
             for (int i = 0; i < SYNC_MASK_WORDS; i += 4) {
                 *reinterpret_cast<int4*>(p.status + SYNC_AMAX_DONE + i) = make_int4(0, 0, 0, 0);
                 *reinterpret_cast<int4*>(p.status + SYNC_ARRIVED + i) = make_int4(0, 0, 0, 0);

@@ -227,7 +227,7 @@ int32_t b200_mla_q_amax(const void *x_bf16, int64_t n, uint32_t *parts_out, void
  * frozen after start-up, code running under a framework that forbids allocator calls in its hot
  * section, or a plain C host that owns no allocator at all.  Same arguments and results as
  * b200_mla_decode, except that `workspace` / `workspace_bytes` are ignored: the split-KV partials,
- * the tile table and the status word live in a B200_MLA_STATIC_WORKSPACE_BYTES array that is part
+ * the table of CTAs and the status word live in a B200_MLA_STATIC_WORKSPACE_BYTES array that is part
  * of the library image on every GPU that loads it (held until the process exits).
  *   - A problem whose b200_mla_workspace_bytes() exceeds that size is refused with
  *     B200_MLA_ERR_TOO_LARGE; nothing is launched.

@@ -138,8 +138,8 @@ def _left(pkg):
     return sum(int(ws[16:20].view(torch.int32)) for ws in submission._workspace_cache.values())
 
 
-# CTAs that do not wait for one another (0 cycles), or not for long: each finds the maximum of Q itself, and those that are late
-# merge what the others had to leave behind.
+# CTAs that do not wait for one another (0 cycles), or not for long: they look at the shares of Q that nobody has looked at, and those
+# that are late merge what the others had to leave behind.
 @pytest.mark.parametrize("kv_format,q_format,heads,lens", [("fp8", "fp8", 16, [900, 0, 97, 2000]), ("mxfp4", "bf16", 32, [4000]),
                                                            ("hybrid", "fp8", 128, [700, 1500, 64]), ("fp8", "bf16", 16, [130] * 300),
                                                            ("fp8", "fp8", 128, [3] * 150 + [6000, 0, 9000] + [3] * 150)])
