@@ -891,16 +891,14 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
                     }
                 };
                 // x = scores relative to the reference maxima (to zero at a sequence's first tile, see nm); from here on the
-                // tile lives in registers and the S buffer goes back.  Where a maximum moves, x is shifted: rounded twice, the first time at
-                // the size it had before, where one FMA with the new maximum rounds once.  That is half an ulp of a score, which the sum over
-                // 18 k-steps carries anyway: errors against 64 bits agree to three digits with those of the FMA up to scores of 158.
+                // tile lives in registers.  Where a maximum moves, x is shifted, so it is rounded twice, the first time relative to the old
+                // maximum: half an ulp of FAR at most.  Beyond FAR the scores are read once more, absolutely (without that the LSE was off by
+                // 3e-5 for a maximum that moves by 2^15 and by 2e-3 for 2^21; 1e-6 so).
+                constexpr float FAR = 256.0f;
                 if (active) {
                     load_scores(ms.nm[sg][nm_cur]);
                     mask_scores();
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&ms.s_empty[sb]);
                 bool recenter = first;
                 if (!first) {
                     float xm = -INFINITY;
@@ -920,26 +918,46 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
                 }
                 unsigned int moved = 0;                           // rows of O to rescale
                 if (recenter) {
-                    const float top = active ? fold_columns<NC, true>(x, lane) : -INFINITY;
-                    if (NC == 32 || !(lane & 1)) ms.red[sg][wv][NC == 32 ? lane : lane >> 1] = top;
-                    named_bar_sync(bar_id, 128);
-                    if (tok < NC) {                               // one thread per query row
-                        const float mx = fmaxf(fmaxf(ms.red[sg][0][tok], ms.red[sg][1][tok]), fmaxf(ms.red[sg][2][tok], ms.red[sg][3][tok]));
-                        const float old = ms.nm[sg][nm_cur][tok];
-                        const float next = mx > (first ? -INFINITY : C::P_SCALE_LOG2) ? old + (C::P_SCALE_LOG2 - mx) : old;
+                    // the tile's maximum of query row tok, in its thread
+                    auto row_max = [&]() {
+                        const float top = active ? fold_columns<NC, true>(x, lane) : -INFINITY;
+                        if (NC == 32 || !(lane & 1)) ms.red[sg][wv][NC == 32 ? lane : lane >> 1] = top;
+                        named_bar_sync(bar_id, 128);
+                        return tok < NC ? fmaxf(fmaxf(ms.red[sg][0][tok], ms.red[sg][1][tok]), fmaxf(ms.red[sg][2][tok], ms.red[sg][3][tok])) : -INFINITY;
+                    };
+                    // x is relative to P_SCALE_LOG2 - base; the row's reference maximum goes from P_SCALE_LOG2 - old to P_SCALE_LOG2 - next
+                    auto move_row = [&](float base, float old, float next) {
                         ms.nm[sg][nm_cur ^ 1][tok] = next;
-                        ms.shift[sg][tok] = next - old;           // what the rounded maximum has moved by
+                        ms.shift[sg][tok] = next - base;
                         ms.fac[sg][tok] = ex2(next - old);
+                    };
+                    float mx = row_max();
+                    if (tok < NC) {                               // one thread per query row
+                        const float old = ms.nm[sg][nm_cur][tok];
+                        move_row(old, old, mx > (first ? -INFINITY : C::P_SCALE_LOG2) ? old + (C::P_SCALE_LOG2 - mx) : old);
+                    }
+                    if (__builtin_expect(named_bar_or(bar_id, 128, !first && tok < NC && mx > FAR), 0)) {
+                        if (tok < NC) ms.shift[sg][tok] = 0.0f;
+                        named_bar_sync(bar_id, 128);
+                        if (active) {
+                            load_scores(ms.shift[sg]);
+                            mask_scores();
+                        }
+                        mx = row_max();
+                        if (tok < NC) {
+                            const float old = ms.nm[sg][nm_cur][tok];
+                            move_row(0.0f, old, fminf(old, C::P_SCALE_LOG2 - mx));
+                        }
+                        named_bar_sync(bar_id, 128);
                     }
                     nm_cur ^= 1;
-                    named_bar_sync(bar_id, 128);
 #pragma unroll
                     for (int c = 0; c < NC; c += 4) {
                         const float4 d4 = *reinterpret_cast<const float4*>(&ms.shift[sg][c]);
                         x[c] += d4.x; x[c + 1] += d4.y; x[c + 2] += d4.z; x[c + 3] += d4.w;
                     }
                     if (!first) {
-                        moved = __ballot_sync(0xffffffffu, lane < NC && ms.shift[sg][lane & (NC - 1)] != 0.0f);
+                        moved = __ballot_sync(0xffffffffu, lane < NC && ms.fac[sg][lane & (NC - 1)] != 1.0f);
 #pragma unroll
                         for (int c = 0; c < NC / 2; c += 2) {
                             const float4 f4 = *reinterpret_cast<const float4*>(&ms.fac[sg][2 * c]);
@@ -947,6 +965,9 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
                         }
                     }
                 }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&ms.s_empty[sb]);
                 uint32_t hi[NC / 4], lo[NC / 4];
                 if (active) {
                     // stored probability = p * 2^P_SCALE_LOG2 * 2^(e_unit - e_run): this token's V bytes are in the frame e_unit, O in e_run

@@ -447,6 +447,34 @@ def test_reference_maxima_that_move_at_most_tiles(pkg, kv_format, q_format, head
         assert float((got - want).norm() / want.norm()) <= 2.0 ** -7
 
 
+# The first tiles' scores lie 2^jump below the later ones': a tile whose maximum is far above the reference is read again, so that its
+# scores keep their last bits.  They agree with 64 bits to some 1e-6; half an ulp of 256, up to which a tile is shifted instead, is 8e-6
+# (5e-6 of the LSE).
+@pytest.mark.parametrize("jump", [5, 9, 13, 15, 17, 21])
+@pytest.mark.parametrize("kv_format,q_format,heads", [("fp8", "bf16", 16), ("fp8", "fp8", 16), ("fp8", "fp8", 64), ("mxfp4", "bf16", 16), ("mxfp4", "bf16", 32),
+                                                      ("mxfp4", "fp8", 64), ("hybrid", "fp8", 64)])
+def test_a_maximum_that_moves_far(pkg, kv_format, q_format, heads, jump):
+    if kv_format == "fp8" and jump > 15:
+        pytest.skip("one scale for the whole cache")
+    n, g = 2000, torch.Generator().manual_seed(jump)
+    kv = torch.randn(n, 1, 576, generator=g)
+    kv[:, 0, :32] = 0.0
+    kv[:512, 0, :32] = -2.0 ** (jump - 1)
+    q = torch.randn(1, heads, 576, generator=g)
+    q[..., :32] = 1.0
+    planes, q = {"fp8": pkg.quantize_fp8, "mxfp4": pkg.quantize_mxfp4, "hybrid": pkg.quantize_hybrid}[kv_format](kv.bfloat16().cuda()), q.bfloat16().cuda()
+    qc, qs = pkg.quantize_q_fp8(q) if q_format == "fp8" else (q, None)
+    keys = mo.dequant_kv(kv_format, tuple(t.cpu() for t in planes)).double().reshape(n, 576)
+    rows = mo.dequant_q(qc.cpu(), None if qs is None else qs.cpu()).double().reshape(heads, 576)
+    scores = rows @ keys.T * 0.0625
+    ip = torch.tensor([0, n], dtype=torch.int32, device="cuda")
+    o, lse = pkg.mla_decode(qc, qs, kv_format, planes, ip, sm_scale=0.0625, return_partial=True, impl="tcgen05", max_ctas=1)
+    assert float((lse.cpu().double().reshape(-1) - torch.logsumexp(scores, 1)).abs().max()) <= 1e-5
+    if kv_format == "fp8":
+        want = torch.softmax(scores, 1) @ keys[:, :512]
+        assert float((o.cpu().double().reshape(heads, 512) - want).norm() / want.norm()) <= 2.0 ** -10
+
+
 def _captured(pkg, data, n=1, stream=None):
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph, stream=stream):
