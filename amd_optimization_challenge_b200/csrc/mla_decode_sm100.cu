@@ -28,9 +28,9 @@
 //        1 QK warp, 1 PV warp (the whole warp runs the loop, one elected lane issues), for a block-scaled cache 2 fetch warps
 //        (the PV warp, or the first fetch warp, searches the CTA's span before that)
 // What bounds it, and microseconds a call before (a kernel per family, maximum of Q and merge as launches of their own, one
-// issuing warp) and now: e4m3 256 x 8192 the HBM rate (264 -> 211), 128 heads over an e4m3 cache the chain load -> QK -> softmax -> PV
-// of two stages (236 -> 80), MXFP4 64 x 8192 the same chain with the conversion in it (96 -> 64), MXFP4 8 x 131072 with two
-// queries and hybrid 128 heads shared memory, conversion and MMA operands alike (214 -> 144, 640 -> 384), e4m3 4 x 1024 latencies
+// issuing warp) and now: e4m3 256 x 8192 the HBM rate (264 -> 213), 128 heads over an e4m3 cache the chain load -> QK -> softmax -> PV
+// of two stages (236 -> 81), MXFP4 64 x 8192 the same chain with the conversion in it (96 -> 65), MXFP4 8 x 131072 with two
+// queries and hybrid 128 heads shared memory, conversion and MMA operands alike (214 -> 146, 640 -> 388), e4m3 4 x 1024 latencies
 // (23.5 -> 10.0 to 10.6).  Long calls vary by 8 % from GPU to GPU.
 // Synchronisation is mbarrier based; every such wait is bounded and on expiry sets a status word.  The two waits for other CTAs
 // are shorter, and who gives up goes on without them and sets no status: see MlaParams::meet_cycles.
@@ -103,7 +103,7 @@ struct Cfg {
     // A probability p (relative to the reference maximum) is stored as 2^P_SCALE_LOG2 p; a score more than RECENTER log2 units above
     // the reference maximum moves it.  2^(P_SCALE_LOG2 + RECENTER) must stay below 448.  The smallest step of the stored pair is
     // 2^-13 with lo / 16 in columns of its own, 2^-9 where lo shares hi's columns (MERGED): there the larger factor keeps the same
-    // 2^-17 below the reference maximum, at the price of moving it at most tiles (48 ragged sequences of 128 heads: 80 us; 85 when
+    // 2^-17 below the reference maximum, at the price of moving it at most tiles (48 ragged sequences of 128 heads: 81 us; 85 when
     // O was rescaled before the probabilities were computed, all of it, and the scores read three times; less with 2^4, but like
     // keys 12 binades down come out 28 % wrong).  Block-scaled caches at 64 rows keep 2^4, i.e. 2^-13.
     static constexpr bool DEEP = MERGED && !XF;
