@@ -1209,12 +1209,9 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
                 tc_fence_after();
                 const uint32_t d_lat = tmem + sb * C::SC, d_rope = d_lat + (C::ROPE_SEP ? NQ : 0);
 #pragma unroll 1
-                for (int j = 0; j < 4; ++j) {
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        umma_f8_elect(d_lat, desc_advance(d_qk_a, st * STAGE_BYTES + j * PANEL_BYTES + k * 32),
-                                      desc_advance(d_qk_b, j * C::Q_PANEL_BYTES + k * 32), IDESC_QK, (j | k) ? 1u : 0u);
-                }
+                for (int j = 0; j < 4; ++j)
+                    umma_f8_x4_elect<0, 32, 32>(d_lat, desc_advance(d_qk_a, st * STAGE_BYTES + j * PANEL_BYTES), desc_advance(d_qk_b, j * C::Q_PANEL_BYTES),
+                                                IDESC_QK, j, 1u);
 #pragma unroll
                 for (int k = 0; k < 2; ++k)
                     umma_f8_elect(d_rope, desc_advance(d_qk_a_rope, st * STAGE_BYTES + k * 32), desc_advance(d_qk_b_rope, k * 32),
@@ -1243,11 +1240,9 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
                 for (int kk = 0; kk < TILE / 32; ++kk) {
 #pragma unroll
                     for (int half = 0; half < (C::MERGED ? 2 : 1); ++half) {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            umma_f8_elect(tmem + C::TMEM_O + j * C::OB, desc_advance(a0, j * PANEL_BYTES + kk * 32 * 128),
-                                          desc_advance(b0, kk * 32 * 16 + half * (N / 16) * C::P_CHUNK_BYTES), IDESC_PV,
-                                          (first && kk == 0 && half == 0) ? 0u : 1u);
+                        const uint32_t acc = !first || kk > 0 || half > 0;
+                        umma_f8_x4_elect<C::OB, PANEL_BYTES, 0>(tmem + C::TMEM_O, desc_advance(a0, kk * 32 * 128),
+                                                                desc_advance(b0, kk * 32 * 16 + half * (N / 16) * C::P_CHUNK_BYTES), IDESC_PV, acc, acc);
                     }
                     umma_commit_elect(&ms.kv_empty[st][kk]);          // these 32 tokens' part of the stage may be refilled
                 }

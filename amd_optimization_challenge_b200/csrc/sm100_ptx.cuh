@@ -157,6 +157,26 @@ __device__ __forceinline__ void umma_f8_elect(uint32_t d_tmem, uint64_t a_desc, 
         "@P1 tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// Four of them behind one election: D, A and B move by D_STEP columns, A_STEP and B_STEP bytes from one to the next; `first` for the first
+// and `rest` for the others: whether D is accumulated into.  The steps are immediates, so that only the first descriptors have to be
+// brought into uniform registers: 16 MMAs of M = 128, K = 32, N = 16 from one idle warp take 918 cycles one by one and 802 so, which is what
+// the tensor core needs for them (977 and 961 with N = 64).
+template <int D_STEP, int A_STEP, int B_STEP>
+__device__ __forceinline__ void umma_f8_x4_elect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t first, uint32_t rest) {
+    static_assert(A_STEP % 16 == 0 && B_STEP % 16 == 0, "descriptors count in 16 bytes");
+    asm volatile(
+        "{\n\t.reg .pred P1, p, q;\n\t.reg .b32 r, d1, d2, d3;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+        "elect.sync r|P1, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "add.u32 d1, %0, %6;\n\tadd.u32 d2, %0, 2*%6;\n\tadd.u32 d3, %0, 3*%6;\n\t"
+        "add.u64 a1, %1, %7;\n\tadd.u64 a2, %1, 2*%7;\n\tadd.u64 a3, %1, 3*%7;\n\t"
+        "add.u64 b1, %2, %8;\n\tadd.u64 b2, %2, 2*%8;\n\tadd.u64 b3, %2, 3*%8;\n\t"
+        "@P1 tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
+        "@P1 tcgen05.mma.cta_group::1.kind::f8f6f4 [d1], a1, b1, %3, q;\n\t"
+        "@P1 tcgen05.mma.cta_group::1.kind::f8f6f4 [d2], a2, b2, %3, q;\n\t"
+        "@P1 tcgen05.mma.cta_group::1.kind::f8f6f4 [d3], a3, b3, %3, q;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(first), "r"(rest), "n"(D_STEP), "n"(A_STEP / 16), "n"(B_STEP / 16) : "memory");
+}
 __device__ __forceinline__ void umma_commit_elect(uint64_t* bar) {
     asm volatile(
         "{\n\t.reg .pred P1;\n\t.reg .b32 r;\n\t"
