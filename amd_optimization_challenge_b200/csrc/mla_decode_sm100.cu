@@ -60,7 +60,7 @@ constexpr int NO_BIT_CYCLES = 20000;      // 10 us, what the CTAs of an ordinary
 enum { MASK_ARRIVED = 0, MASK_LATE_ARRIVED = 1, MASK_LATE_LEFT = 2 };      // see Misc::mask
 
 struct Misc {
-    uint64_t kv_full[NS_MAX], kv_empty[NS_MAX][4], s_full[2], s_empty[2], p_full[2], p_empty[2], q_full, o_free;
+    uint64_t kv_full[NS_MAX], kv_empty[NS_MAX][4], s_full[2], s_empty[2], p_full[NS_MAX], p_empty[NS_MAX], q_full, o_free;
     uint64_t raw_full[RAW_MAX], raw_empty[RAW_MAX];
     int raw_slot[RAW_MAX][UNIT_TOK];      // cache rows of the unit in each landing buffer
     uint32_t tmem_base;
@@ -110,7 +110,7 @@ struct Cfg {
     static constexpr float P_SCALE_LOG2 = DEEP ? 8.0f : 4.0f, RECENTER = DEEP ? 0.75f : 4.0f;
     static constexpr int P_CHUNK_BYTES = TILE * 16;               // 16 columns x TILE tokens
     static constexpr int P_BUF_BYTES = (2 * N / 16) * P_CHUNK_BYTES;
-    static constexpr int P_BUFS = XF && N > 16 ? 1 : 2;           // single where the landing buffers need the room
+    static constexpr int P_BUFS = XF && N > 16 ? 1 : NS;          // single where the landing buffers need the room
     static constexpr int Q_PANEL_BYTES = NQ * 128;
     static constexpr int Q_BYTES = NQ * QK_DIM;                   // four 128B-swizzled panels and one 64B-swizzled
     // Landing buffer of one unit: 16 code rows (see raw_chunk), then 32 bytes around each E8M0 row.
@@ -579,8 +579,8 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&ms.s_full[i], 1); mbar_init(&ms.s_empty[i], SW);
-            mbar_init(&ms.p_full[i], SW); mbar_init(&ms.p_empty[i], 1);
         }
+        for (int i = 0; i < P_BUFS; ++i) { mbar_init(&ms.p_full[i], SW); mbar_init(&ms.p_empty[i], 1); }
         for (int i = 0; i < C::NBUF; ++i) { mbar_init(&ms.raw_full[i], 33); mbar_init(&ms.raw_empty[i], 1); }
         mbar_init(&ms.q_full, SW);
         mbar_init(&ms.o_free, SW);
@@ -837,6 +837,11 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
                     qk_base = p.sm_scale * LOG2E * q_scale;
                 }
                 const int pos_first = (t_begin + g - wk.t0) * TILE;
+                // P(g) may overwrite its buffer once the PV that read it last has completed.  With as many buffers as stages that is the PV that
+                // gives back the stage of this tile, which S waits for as well: looked at here it costs nothing, 130 cycles of the chain
+                // behind S otherwise.
+                const int pb = g % P_BUFS;
+                if (P_BUFS == NS) mbar_wait(&ms.p_empty[pb], g / P_BUFS - 1, abort_flag);
                 mbar_wait(&ms.s_full[sb], g / 2, abort_flag);
                 tc_fence_after();
                 // exponent frames: e_unit of this thread's token, e_tile = the largest of the tile's units
@@ -992,9 +997,7 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
                         lo[q4] = pack_e4m3x4(p0, p1, p2, p3);
                     }
                 }
-                // P(g) may overwrite its buffer once the PV that read it last has completed
-                const int pb = g % P_BUFS;
-                mbar_wait(&ms.p_empty[pb], g / P_BUFS - 1, abort_flag);
+                if (P_BUFS < NS) mbar_wait(&ms.p_empty[pb], g / P_BUFS - 1, abort_flag);
                 if (active) {
                     uint8_t* pbuf = smem + C::OFF_P + pb * C::P_BUF_BYTES + (col0 / 16) * C::P_CHUNK_BYTES + tok * 16;
 #pragma unroll
