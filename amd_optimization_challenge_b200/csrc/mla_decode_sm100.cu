@@ -1091,20 +1091,14 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
                     if (use_tma) {
                         mbar_arrive_expect_tx_elect(&ms.kv_full[st], UNIT_TOK * QK_DIM);
                         if (box) {
-                            const int r0 = (int)__shfl_sync(0xffffffffu, slot, 0);
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) tma_load_2d_elect(lat + i * PANEL_BYTES, &maps.lat_box, 128 * i, r0, &ms.kv_full[st], pol);
-                            tma_load_2d_elect(rope, &maps.rope_box, 512, r0, &ms.kv_full[st], pol);
+                            tma_rows_box_elect<PANEL_BYTES>(lat, rope, &maps.lat_box, &maps.rope_box, (int)__shfl_sync(0xffffffffu, slot, 0), &ms.kv_full[st], pol);
                         } else {
 #pragma unroll 1
                             for (int q = 0; q < 4; ++q) {
                                 int r[4];
 #pragma unroll
                                 for (int i = 0; i < 4; ++i) r[i] = (int)__shfl_sync(0xffffffffu, slot, 4 * q + i);
-#pragma unroll
-                                for (int i = 0; i < 4; ++i)
-                                    tma_gather4_2d_elect(lat + i * PANEL_BYTES + q * 512, &maps.lat, 128 * i, r[0], r[1], r[2], r[3], &ms.kv_full[st], pol);
-                                tma_gather4_2d_elect(rope + q * 256, &maps.rope, 512, r[0], r[1], r[2], r[3], &ms.kv_full[st], pol);
+                                tma_rows_gather4_elect<PANEL_BYTES>(lat + q * 512, rope + q * 256, &maps.lat, &maps.rope, r[0], r[1], r[2], r[3], &ms.kv_full[st], pol);
                             }
                         }
                     } else {                                          // no tensor maps (driver entry point missing): 16-byte copies

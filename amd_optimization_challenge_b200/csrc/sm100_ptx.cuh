@@ -58,21 +58,40 @@ __device__ __forceinline__ void mbar_arrive_expect_tx_elect(uint64_t* bar, uint3
                  "@P1 mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}"
                  ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-// Tiled 2-D TMA load of one box (as the tensor map defines it) whose first element is (x, y); x is in elements of the map
-// and must be a multiple of 16 bytes.  Completion is counted in bytes on `bar`.  `policy`: see l2_evict_first_policy.
-__device__ __forceinline__ void tma_load_2d_elect(uint32_t dst_smem, const void* tmap, int x, int y, uint64_t* bar, uint64_t policy) {
-    asm volatile("{\n\t.reg .pred P1;\n\t.reg .b32 e;\n\telect.sync e|P1, 0xffffffff;\n\t"
-                 "@P1 cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;\n\t}"
-                 ::"r"(dst_smem), "l"(tmap), "r"(x), "r"(y), "r"(smem_u32(bar)), "l"(policy) : "memory");
+// Tiled 2-D TMA loads of rows of 576 bytes: their four 128-byte columns to `lat` and PANEL bytes on from one to the next, the last 64 bytes
+// to `rope`, by the two maps' boxes (PANEL and the columns x are multiples of 16 bytes).  Completion is counted in bytes on `bar`.  `policy`: see
+// l2_evict_first_policy.  All five behind one election: with one each, and every operand brought into uniform registers each time, the boxes of a
+// unit of 16 rows took 600 cycles.
+// The box whose first row is y.
+template <int PANEL>
+__device__ __forceinline__ void tma_rows_box_elect(uint32_t lat, uint32_t rope, const void* lat_map, const void* rope_map, int y, uint64_t* bar, uint64_t policy) {
+    static_assert(PANEL % 16 == 0, "TMA destinations");
+    asm volatile(
+        "{\n\t.reg .pred P1;\n\t.reg .b32 e, d1, d2, d3, x0, x1, x2, x3, x4;\n\telect.sync e|P1, 0xffffffff;\n\t"
+        "mov.b32 x0, 0;\n\tmov.b32 x1, 128;\n\tmov.b32 x2, 256;\n\tmov.b32 x3, 384;\n\tmov.b32 x4, 512;\n\t"
+        "add.u32 d1, %0, %7;\n\tadd.u32 d2, %0, 2*%7;\n\tadd.u32 d3, %0, 3*%7;\n\t"
+        "@P1 cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%2, {x0, %4}], [%5], %6;\n\t"
+        "@P1 cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [d1], [%2, {x1, %4}], [%5], %6;\n\t"
+        "@P1 cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [d2], [%2, {x2, %4}], [%5], %6;\n\t"
+        "@P1 cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [d3], [%2, {x3, %4}], [%5], %6;\n\t"
+        "@P1 cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%1], [%3, {x4, %4}], [%5], %6;\n\t}"
+        ::"r"(lat), "r"(rope), "l"(lat_map), "l"(rope_map), "r"(y), "r"(smem_u32(bar)), "l"(policy), "n"(PANEL) : "memory");
 }
-// Tiled 2-D TMA gather of FOUR rows (y0..y3, any order, any distance) of the map's tensor, `box width` bytes each starting
-// at x (a multiple of 16 bytes), into four consecutive rows at dst_smem; the map's box is {width, 1}.  The swizzle of the
-// map is applied as for an ordinary tile.  Completion is counted in bytes (4 x width) on `bar`.  This GPU's memory only.
-__device__ __forceinline__ void tma_gather4_2d_elect(uint32_t dst_smem, const void* tmap, int x, int y0, int y1, int y2, int y3, uint64_t* bar,
-                                                     uint64_t policy) {
-    asm volatile("{\n\t.reg .pred P1;\n\t.reg .b32 e;\n\telect.sync e|P1, 0xffffffff;\n\t"
-                 "@P1 cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4, %5, %6}], [%7], %8;\n\t}"
-                 ::"r"(dst_smem), "l"(tmap), "r"(x), "r"(y0), "r"(y1), "r"(y2), "r"(y3), "r"(smem_u32(bar)), "l"(policy) : "memory");
+// FOUR rows (y0..y3, any order, any distance), one below the other; the maps' boxes are one row high.  This GPU's memory only.
+template <int PANEL>
+__device__ __forceinline__ void tma_rows_gather4_elect(uint32_t lat, uint32_t rope, const void* lat_map, const void* rope_map, int y0, int y1, int y2, int y3,
+                                                       uint64_t* bar, uint64_t policy) {
+    static_assert(PANEL % 16 == 0, "TMA destinations");
+    asm volatile(
+        "{\n\t.reg .pred P1;\n\t.reg .b32 e, d1, d2, d3, x0, x1, x2, x3, x4;\n\telect.sync e|P1, 0xffffffff;\n\t"
+        "mov.b32 x0, 0;\n\tmov.b32 x1, 128;\n\tmov.b32 x2, 256;\n\tmov.b32 x3, 384;\n\tmov.b32 x4, 512;\n\t"
+        "add.u32 d1, %0, %10;\n\tadd.u32 d2, %0, 2*%10;\n\tadd.u32 d3, %0, 3*%10;\n\t"
+        "@P1 cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%2, {x0, %4, %5, %6, %7}], [%8], %9;\n\t"
+        "@P1 cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes.L2::cache_hint [d1], [%2, {x1, %4, %5, %6, %7}], [%8], %9;\n\t"
+        "@P1 cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes.L2::cache_hint [d2], [%2, {x2, %4, %5, %6, %7}], [%8], %9;\n\t"
+        "@P1 cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes.L2::cache_hint [d3], [%2, {x3, %4, %5, %6, %7}], [%8], %9;\n\t"
+        "@P1 cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes.L2::cache_hint [%1], [%3, {x4, %4, %5, %6, %7}], [%8], %9;\n\t}"
+        ::"r"(lat), "r"(rope), "l"(lat_map), "l"(rope_map), "r"(y0), "r"(y1), "r"(y2), "r"(y3), "r"(smem_u32(bar)), "l"(policy), "n"(PANEL) : "memory");
 }
 // Policy word for data that is read once (the cache rows): its lines are the first to leave L2, so the streaming
 // megabytes do not push out what every launch needs again - the kernels' code, Q, the page table.
