@@ -1093,7 +1093,7 @@ mla_decode_sm100_kernel(const __grid_constant__ MlaParams p, const __grid_consta
                         if (box) {
                             tma_rows_box_elect<PANEL_BYTES>(lat, rope, &maps.lat_box, &maps.rope_box, (int)__shfl_sync(0xffffffffu, slot, 0), &ms.kv_full[st], pol);
                         } else {
-#pragma unroll 1
+#pragma unroll
                             for (int q = 0; q < 4; ++q) {
                                 int r[4];
 #pragma unroll
