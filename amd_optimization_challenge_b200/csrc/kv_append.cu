@@ -34,7 +34,7 @@ struct AppendParams {
 };
 
 constexpr int THREADS = 288;
-constexpr int RESIDENT = 7;                                         // blocks on an SM
+constexpr int resident(bool ahead) { return ahead ? 4 : 7; }        // blocks on an SM
 constexpr int vectors(int kv_format) { return kv_format == KV_E4M3 ? 2 : 1; }                   // of eight elements per thread
 constexpr int block_rows(int kv_format) { return THREADS * 8 * vectors(kv_format) / QK_DIM; }   // rows a block covers at a time
 
@@ -110,9 +110,9 @@ __device__ __forceinline__ uint32_t quant_mxfp4x8(const uint4& v, uint8_t& scale
 // Instructions bound it next to HBM, so a thread keeps pointers and advances them, and an e4m3 thread has two vectors: 500000
 // rows into an e4m3 cache (864 MB moved) 158 us with listed slots and 146 without, 205 and 176 with one vector and 64-bit
 // products per row.  A block's first loads are issued before anything that waits for the scale.  Seven resident blocks, one step
-// in flight each: two steps spill registers (16384 rows, e4m3: 6.3 us from one launch to the next with one step, 7.9 with two).
-template <int KVFMT, bool LISTED>
-__global__ void __launch_bounds__(THREADS, RESIDENT) kv_append_kernel(const AppendParams p) {
+// in flight each; with AHEAD four blocks, whose next rows are on their way while a step is converted and stored (see launch_format).
+template <int KVFMT, bool LISTED, bool AHEAD>
+__global__ void __launch_bounds__(THREADS, resident(AHEAD)) kv_append_kernel(const AppendParams p) {
     pdl_wait();
     constexpr int VEC = vectors(KVFMT), CHUNKS = QK_DIM / 8 / VEC, STEP = block_rows(KVFMT);
     const int lead = p.write_status;
@@ -145,9 +145,9 @@ __global__ void __launch_bounds__(THREADS, RESIDENT) kv_append_kernel(const Appe
     const int* list = p.slots + row0 + sub;
     long long to = p.base_slot + row0 + sub;                                          // row of the cache, where no slots are listed
     long long left = p.n - row0;                                                      // rows from the block's first one on
-    uint4 v[VEC];
-    unsigned int slot;
-    auto fetch = [&]() {
+    uint4 v[VEC], next[VEC];
+    unsigned int slot, next_slot;
+    auto fetch = [&](uint4 (&v)[VEC], unsigned int& slot) {
         slot = 0xffffffffu;
 #pragma unroll
         for (int k = 0; k < VEC; ++k) v[k] = make_uint4(0u, 0u, 0u, 0u);
@@ -160,11 +160,14 @@ __global__ void __launch_bounds__(THREADS, RESIDENT) kv_append_kernel(const Appe
         list += hop;
     };
     const float scale = KVFMT != KV_MXFP4 ? __ldcg(p.scale) : 1.0f;
-    fetch();
+    fetch(v, slot);
     const float rscale = __frcp_rn(scale);
     const unsigned int general = general_from(rscale);
     for (;;) {                                                                        // the same number of steps for the whole block
-        const bool mine = sub < left, ok = LISTED ? slot < top : mine;                // nothing is written elsewhere
+        const bool mine = sub < left;
+        left -= hop;
+        if (AHEAD && left > 0) fetch(next, next_slot);
+        const bool ok = LISTED ? slot < top : mine;                // nothing is written elsewhere
         if (LISTED) {
             if (mine && !ok && !p.write_status) *p.bad = 1;
             to = (long long)slot;
@@ -185,20 +188,36 @@ __global__ void __launch_bounds__(THREADS, RESIDENT) kv_append_kernel(const Appe
                 if ((chunk & 3) == 0) p.bs[to * p.bs_stride + (chunk >> 2)] = sb;
             }
         }
-        left -= hop;
         if (left <= 0) break;
         to += hop;
-        fetch();
+        if constexpr (AHEAD) {
+            slot = next_slot;
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) v[k] = next[k];
+        } else {
+            fetch(v, slot);
+        }
     }
 }
 
 // Up to eight steps per block of a single resident wave the blocks stay and loop (16384 rows, e4m3: 6.3 us, 7.8 with a wave
 // more); beyond that four waves even out what the blocks take (131072 rows: 38.4 us, 44.8 with one).
+// Listed rows of an e4m3 cache have the slot's load in front of each step; where a wave of seven blocks takes two steps at most, they are
+// fetched a step ahead by four (us, without and with: 9000 rows 4.83 and 4.66, 12000 5.00 and 4.77, 16384 6.65 and 6.36).  Beyond that there are
+// bytes enough in flight and the smaller wave is slower (24000 rows 9.57 and 10.55, 66000 24.0 and 25.4).  The other formats and
+// unlisted rows gain nothing (e4m3, 16384 rows 6.12 and 6.13).
+template <int KVFMT, bool LISTED, bool AHEAD>
+cudaError_t launch_waves(const AppendParams& p, long long steps, long long cap, cudaStream_t stream) {
+    const unsigned int blocks = (unsigned int)(steps < cap ? steps : cap) + (unsigned int)p.write_status;
+    return launch_pdl(kv_append_kernel<KVFMT, LISTED, AHEAD>, blocks, THREADS, 0, stream, p);
+}
 template <int KVFMT>
 cudaError_t launch_format(const AppendParams& p, cudaStream_t stream) {
-    const long long wave = 148 * RESIDENT, steps = (p.n + block_rows(KVFMT) - 1) / block_rows(KVFMT), cap = steps <= 8 * wave ? wave : 4 * wave;
-    const unsigned int blocks = (unsigned int)(steps < cap ? steps : cap) + (unsigned int)p.write_status;
-    return launch_pdl(p.slots ? kv_append_kernel<KVFMT, true> : kv_append_kernel<KVFMT, false>, blocks, THREADS, 0, stream, p);
+    const long long wave = 148 * resident(false), steps = (p.n + block_rows(KVFMT) - 1) / block_rows(KVFMT);
+    if (!p.slots) return launch_waves<KVFMT, false, false>(p, steps, steps <= 8 * wave ? wave : 4 * wave, stream);
+    constexpr bool AHEAD = KVFMT == KV_E4M3;
+    if (AHEAD && steps <= 2 * wave) return launch_waves<KVFMT, true, AHEAD>(p, steps, 148 * resident(AHEAD), stream);
+    return launch_waves<KVFMT, true, false>(p, steps, steps <= 8 * wave ? wave : 4 * wave, stream);
 }
 
 }  // namespace

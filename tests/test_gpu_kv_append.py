@@ -79,6 +79,28 @@ def test_append_matches_host_quantisers_at_shuffled_slots(pkg):
     assert int(st) == 1
 
 
+@pytest.mark.parametrize("n", [1, 9, 4736, 4737, 9473, 16576, 16577])
+def test_listed_e4m3_rows_around_the_steps_of_a_wave(pkg, n):
+    """Listed rows (fetched a step ahead up to 16576 of them, a wave of 4736 at a time) against unlisted ones, bytes of the same rows in
+    another order; single slots outside the cache, the first and the last of the list among them, are left out and reported."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rows = torch.randn(n, 576, dtype=torch.bfloat16, generator=g, device="cuda")
+    scale = torch.full((1,), 4.5 / 448, device="cuda")
+    want = torch.zeros(n, 576, dtype=torch.uint8, device="cuda")
+    assert int(pkg.kv_append(rows, "fp8", (want, scale))) == 0
+    slots = torch.randperm(n + 3, generator=g, device="cuda")[:n].to(torch.int32)
+    for outside in ([], sorted({0, n // 2, n - 1})):
+        got = torch.full((n + 3, 576), 0xEE, dtype=torch.uint8, device="cuda")
+        listed = slots.clone()
+        listed[outside] = n + 3
+        status = pkg.kv_append(rows, "fp8", (got, scale), slots=listed)
+        expected = torch.full((n + 3, 576), 0xEE, dtype=torch.uint8, device="cuda")
+        inside = listed < n + 3
+        expected[listed[inside].long()] = want[inside]
+        assert torch.equal(got, expected)
+        assert int(status) == (1 if outside else 0)
+
+
 @pytest.mark.parametrize("kv_format,q_format", [("fp8", "fp8"), ("mxfp4", "bf16"), ("hybrid", "fp8")])
 def test_decode_of_a_device_filled_cache(pkg, kv_format, q_format):
     """Append in two batches (as prefill + decode steps would), then decode through custom_kernel."""
