@@ -28,9 +28,9 @@
 //        1 QK warp, 1 PV warp (the whole warp runs the loop, one elected lane issues), for a block-scaled cache 2 fetch warps
 //        (the PV warp, or the first fetch warp, searches the CTA's span before that)
 // What bounds it, and microseconds a call before (a kernel per family, maximum of Q and merge as launches of their own, one
-// issuing warp) and now: e4m3 256 x 8192 the HBM rate (264 -> 213), 128 heads over an e4m3 cache the chain load -> QK -> softmax -> PV
-// of two stages (236 -> 81), MXFP4 64 x 8192 the same chain with the conversion in it (96 -> 65), MXFP4 8 x 131072 with two
-// queries and hybrid 128 heads shared memory, conversion and MMA operands alike (214 -> 146, 640 -> 388), e4m3 4 x 1024 latencies
+// issuing warp) and now: e4m3 256 x 8192 the HBM rate (264 -> 210), 128 heads over an e4m3 cache the chain load -> QK -> softmax -> PV
+// of two stages (236 -> 80), MXFP4 64 x 8192 the same chain with the conversion in it (96 -> 65), MXFP4 8 x 131072 with two
+// queries and hybrid 128 heads that chain and shared memory, conversion and MMA operands alike (214 -> 147, 640 -> 390), e4m3 4 x 1024 latencies
 // (23.5 -> 10.0 to 10.6).  Long calls vary by 8 % from GPU to GPU.
 // Synchronisation is mbarrier based; every such wait is bounded and on expiry sets a status word.  The two waits for other CTAs
 // are shorter, and who gives up goes on without them and sets no status: see MlaParams::meet_cycles.
