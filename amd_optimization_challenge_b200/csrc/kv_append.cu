@@ -206,18 +206,22 @@ __global__ void __launch_bounds__(THREADS, resident(AHEAD)) kv_append_kernel(con
 // fetched a step ahead by four (us, without and with: 9000 rows 4.83 and 4.66, 12000 5.00 and 4.77, 16384 6.65 and 6.36).  Beyond that there are
 // bytes enough in flight and the smaller wave is slower (24000 rows 9.57 and 10.55, 66000 24.0 and 25.4).  The other formats and
 // unlisted rows gain nothing (e4m3, 16384 rows 6.12 and 6.13).
+// The status block counts as one of a single wave's: one block more waits for another to leave and then takes all of its steps behind
+// them (us with rows in HBM, a block more and not: listed e4m3 16384 rows 7.33 and 6.96, 24000 rows by the kernel that fetches ahead 10.3
+// and 9.0; listed MXFP4 16384 rows 7.09 and 6.76).
 template <int KVFMT, bool LISTED, bool AHEAD>
-cudaError_t launch_waves(const AppendParams& p, long long steps, long long cap, cudaStream_t stream) {
-    const unsigned int blocks = (unsigned int)(steps < cap ? steps : cap) + (unsigned int)p.write_status;
-    return launch_pdl(kv_append_kernel<KVFMT, LISTED, AHEAD>, blocks, THREADS, 0, stream, p);
+cudaError_t launch_waves(const AppendParams& p, long long steps, int waves, cudaStream_t stream) {
+    const long long blocks = waves * 148 * resident(AHEAD) - (waves == 1 ? p.write_status : 0);
+    return launch_pdl(kv_append_kernel<KVFMT, LISTED, AHEAD>, (unsigned int)((steps < blocks ? steps : blocks) + p.write_status), THREADS, 0, stream, p);
 }
 template <int KVFMT>
 cudaError_t launch_format(const AppendParams& p, cudaStream_t stream) {
     const long long wave = 148 * resident(false), steps = (p.n + block_rows(KVFMT) - 1) / block_rows(KVFMT);
-    if (!p.slots) return launch_waves<KVFMT, false, false>(p, steps, steps <= 8 * wave ? wave : 4 * wave, stream);
+    const int waves = steps <= 8 * wave ? 1 : 4;
+    if (!p.slots) return launch_waves<KVFMT, false, false>(p, steps, waves, stream);
     constexpr bool AHEAD = KVFMT == KV_E4M3;
-    if (AHEAD && steps <= 2 * wave) return launch_waves<KVFMT, true, AHEAD>(p, steps, 148 * resident(AHEAD), stream);
-    return launch_waves<KVFMT, true, false>(p, steps, steps <= 8 * wave ? wave : 4 * wave, stream);
+    if (AHEAD && steps <= 2 * wave) return launch_waves<KVFMT, true, AHEAD>(p, steps, 1, stream);
+    return launch_waves<KVFMT, true, false>(p, steps, waves, stream);
 }
 
 }  // namespace

@@ -101,6 +101,44 @@ def test_listed_e4m3_rows_around_the_steps_of_a_wave(pkg, n):
         assert int(status) == (1 if outside else 0)
 
 
+def _captured_launch(call):
+    """Blocks of the one kernel that `call` launches, blocks of it that an SM holds, and the number of SMs."""
+    from cuda.bindings import driver
+    def ok(result):
+        assert result[0] == driver.CUresult.CUDA_SUCCESS, result[0]
+        return result[1:]
+    call()                                                       # the first call to a cache is checked in Python and zeroes its status word
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        keep = call()
+    handle = driver.CUgraph(graph.raw_cuda_graph())
+    _, count = ok(driver.cuGraphGetNodes(handle))
+    nodes, _ = ok(driver.cuGraphGetNodes(handle, count))
+    kernels = [n for n in nodes if ok(driver.cuGraphNodeGetType(n))[0] == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL]
+    assert len(kernels) == 1
+    params, = ok(driver.cuGraphKernelNodeGetParams(kernels[0]))
+    func = params.func if int(params.func) else ok(driver.cuKernelGetFunction(params.kern))[0]
+    held, = ok(driver.cuOccupancyMaxActiveBlocksPerMultiprocessor(func, params.blockDimX, params.sharedMemBytes))
+    del keep
+    return params.gridDimX, held, torch.cuda.get_device_properties(0).multi_processor_count
+
+
+# steps of 8 rows for an e4m3 cache, of 4 for the others; sizes of one step per block, of several, and the edges between
+@pytest.mark.parametrize("kv_format,n,listed", [("fp8", 1, True), ("fp8", 4736, True), ("fp8", 4737, True), ("fp8", 9473, True), ("fp8", 16576, True), ("fp8", 16577, True),
+                                                ("fp8", 8288, False), ("fp8", 8289, False), ("mxfp4", 4144, True), ("mxfp4", 4145, True), ("hybrid", 16384, True)])
+def test_blocks_that_stay_for_several_steps_are_on_the_gpu_together(pkg, kv_format, n, listed):
+    """The block that writes the status word counts: one too many would begin when another has ended and take its steps alone."""
+    u8 = dict(dtype=torch.uint8, device="cuda")
+    scale = torch.full((1,), 0.01, device="cuda")
+    planes = {"fp8": lambda: (torch.empty(n, 576, **u8), scale), "mxfp4": lambda: (torch.empty(n, 288, **u8), torch.empty(n, 18, **u8)),
+              "hybrid": lambda: (torch.empty(n, 256, **u8), torch.empty(n, 16, **u8), torch.empty(n, 64, **u8), scale)}[kv_format]()
+    rows = torch.zeros(n, 576, dtype=torch.bfloat16, device="cuda")
+    where = dict(slots=torch.arange(n, dtype=torch.int32, device="cuda")) if listed else {}
+    grid, held, sms = _captured_launch(lambda: pkg.kv_append(rows, kv_format, planes, **where))
+    assert 1 < grid <= held * sms
+    assert grid <= -(-n // (8 if kv_format == "fp8" else 4)) + 1
+
+
 @pytest.mark.parametrize("kv_format,q_format", [("fp8", "fp8"), ("mxfp4", "bf16"), ("hybrid", "fp8")])
 def test_decode_of_a_device_filled_cache(pkg, kv_format, q_format):
     """Append in two batches (as prefill + decode steps would), then decode through custom_kernel."""
