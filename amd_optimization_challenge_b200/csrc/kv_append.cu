@@ -109,8 +109,9 @@ __device__ __forceinline__ uint32_t quant_mxfp4x8(const uint4& v, uint8_t& scale
 
 // Instructions bound it next to HBM, so a thread keeps pointers and advances them, and an e4m3 thread has two vectors: 500000
 // rows into an e4m3 cache (864 MB moved) 158 us with listed slots and 146 without, 205 and 176 with one vector and 64-bit
-// products per row.  A block's first loads are issued before anything that waits for the scale.  Seven resident blocks, one step
-// in flight each; with AHEAD four blocks, whose next rows are on their way while a step is converted and stored (see launch_format).
+// products per row (all with seven blocks).  A block's first loads are issued before anything that waits for the scale.  Seven resident blocks of
+// 32 registers a thread, one step in flight each; with AHEAD four, whose next rows are on their way while a step is converted and
+// stored (see launch_format): that takes 51 registers, and 56 are given out.
 template <int KVFMT, bool LISTED, bool AHEAD>
 __global__ void __launch_bounds__(THREADS, resident(AHEAD)) kv_append_kernel(const AppendParams p) {
     pdl_wait();
@@ -200,28 +201,30 @@ __global__ void __launch_bounds__(THREADS, resident(AHEAD)) kv_append_kernel(con
     }
 }
 
-// Up to eight steps per block of a single resident wave the blocks stay and loop (16384 rows, e4m3: 6.3 us, 7.8 with a wave
-// more); beyond that four waves even out what the blocks take (131072 rows: 38.4 us, 44.8 with one).
-// Listed rows of an e4m3 cache have the slot's load in front of each step; where a wave of seven blocks takes two steps at most, they are
-// fetched a step ahead by four (us, without and with: 9000 rows 4.83 and 4.66, 12000 5.00 and 4.77, 16384 6.65 and 6.36).  Beyond that there are
-// bytes enough in flight and the smaller wave is slower (24000 rows 9.57 and 10.55, 66000 24.0 and 25.4).  The other formats and
-// unlisted rows gain nothing (e4m3, 16384 rows 6.12 and 6.13).
 // The status block counts as one of a single wave's: one block more waits for another to leave and then takes all of its steps behind
-// them (us with rows in HBM, a block more and not: listed e4m3 16384 rows 7.33 and 6.96, 24000 rows by the kernel that fetches ahead 10.3
-// and 9.0; listed MXFP4 16384 rows 7.09 and 6.76).
+// them (us with rows in HBM, a block more and not: listed e4m3 16384 rows 7.33 and 6.96, 24000 rows 10.3 and 9.0; listed MXFP4 16384 rows
+// 7.09 and 6.76).
 template <int KVFMT, bool LISTED, bool AHEAD>
 cudaError_t launch_waves(const AppendParams& p, long long steps, int waves, cudaStream_t stream) {
     const long long blocks = waves * 148 * resident(AHEAD) - (waves == 1 ? p.write_status : 0);
     return launch_pdl(kv_append_kernel<KVFMT, LISTED, AHEAD>, (unsigned int)((steps < blocks ? steps : blocks) + p.write_status), THREADS, 0, stream, p);
 }
+// Seven blocks on an SM: up to eight steps per block of a single wave the blocks stay and loop (unlisted e4m3, 16384 rows 5.7 us, 7.2 with
+// a second wave); beyond that four waves even out what the blocks take (131072 rows 40.3 us, 44.5 with one).
+// Listed rows of an e4m3 cache have the slot's load in front of each step: one wave of four blocks that fetch a step ahead takes them.  Up to six
+// blocks on an SM have one step each, nothing to fetch ahead, and more bytes in flight without (us, seven blocks and four ahead, rows in
+// L2 | in HBM: 512 rows 1.47 and 1.56 | 2.04 and 2.09, 4736 2.85 and 3.03 | 3.40 and 3.65, 6000 3.50 and 3.28 | 3.95 and 4.28,
+// 7104 3.95 and 3.52 | 4.44 and 4.49).  Above that it is the faster one, but for two to three steps a block of rows in HBM (7400
+// 4.18 and 3.52 | 4.59 and 4.51, 9000 4.63 and 3.93 | 5.00 and 4.86, 12000 4.86 and 4.55 | 5.61 and 5.82, 16384 6.06 and 5.61 | 6.98 and
+// 6.98, 24000 7.86 and 7.43 | 8.97 and 8.99, 50000 18.0 and 16.4 | 18.3 and 16.5, 131072 41.0 and 40.4 | 40.6 and 40.5, 500000
+// 157 and 150 | 157 and 150).
 template <int KVFMT>
 cudaError_t launch_format(const AppendParams& p, cudaStream_t stream) {
-    const long long wave = 148 * resident(false), steps = (p.n + block_rows(KVFMT) - 1) / block_rows(KVFMT);
-    const int waves = steps <= 8 * wave ? 1 : 4;
-    if (!p.slots) return launch_waves<KVFMT, false, false>(p, steps, waves, stream);
+    const long long steps = (p.n + block_rows(KVFMT) - 1) / block_rows(KVFMT);
     constexpr bool AHEAD = KVFMT == KV_E4M3;
-    if (AHEAD && steps <= 2 * wave) return launch_waves<KVFMT, true, AHEAD>(p, steps, 1, stream);
-    return launch_waves<KVFMT, true, false>(p, steps, waves, stream);
+    if (AHEAD && p.slots && steps > 148 * 6) return launch_waves<KVFMT, true, AHEAD>(p, steps, 1, stream);
+    const int waves = steps <= 8 * 148 * resident(false) ? 1 : 4;
+    return p.slots ? launch_waves<KVFMT, true, false>(p, steps, waves, stream) : launch_waves<KVFMT, false, false>(p, steps, waves, stream);
 }
 
 }  // namespace
