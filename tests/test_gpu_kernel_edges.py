@@ -18,7 +18,8 @@ def pkg():
     return pkg
 
 
-# a block covers 4 rows at a time and holds 2 such steps; 148 * 7 blocks are one step of the grid (4144 rows)
+# a block covers 8 rows of an e4m3 cache at a time and 4 of the others; 148 * 7 blocks, the one for the status word among them, are one step of
+# the grid (8280 and 4140 rows)
 @pytest.mark.parametrize("n", [1, 3, 4, 5, 4143, 4145, 8289])
 @pytest.mark.parametrize("listed", [False, True])
 def test_append_rows_around_the_steps_of_block_and_grid(pkg, n, listed):
@@ -665,7 +666,32 @@ def test_append_casts_special_values_as_the_division_does(pkg, scale):
     assert torch.equal(got[~nan], want[~nan]) and bool(((got[nan] & 0x7f) == 0x7f).all())
 
 
-# e4m3: 8 rows a block and step, 4 else; 1036 blocks stay for up to eight steps, then there are 4144
+# The same where rows are fetched a step ahead: listed, beyond 7104 of them, 4728 a step of the grid; special rows in each of three
+# steps, and a slot list that begins on and off a 16-byte boundary.
+@pytest.mark.parametrize("scale,off", [(0.01, 0), (1.0, 3), (2.0 ** -100, 1), (2.0 ** 100, 2)])
+def test_append_of_listed_rows_casts_special_values_in_every_step(pkg, scale, off):
+    n, pool, g = 9500, 9600, torch.Generator().manual_seed(off)
+    rows = (torch.randn(n, 576, generator=g) * torch.exp2(torch.randint(-40, 40, (n, 576), generator=g).float())).bfloat16()
+    for r in (0, 4728, 9456):
+        rows[r + 3, 8], rows[r + 4, 15], rows[r + 5, 16] = float("inf"), float("-inf"), 3.0e38
+        rows[r + 6, 1], rows[r + 7, 9], rows[r + 8, 575] = -3.0e38, float("nan"), -0.0
+    q = (rows.float() / torch.tensor(scale)).bfloat16().float()
+    want = q.clamp(-448.0, 448.0).to(torch.float8_e4m3fn).view(torch.uint8)
+    slots = torch.randperm(pool, generator=g)[:n]
+    around = torch.full((n + 8,), -7, dtype=torch.int32, device="cuda")
+    listed = around[off:off + n]
+    listed.copy_(slots)
+    plane = torch.full((pool, 576), 0xEE, dtype=torch.uint8, device="cuda")
+    assert int(pkg.kv_append(rows.cuda(), "fp8", (plane, torch.tensor([scale]).cuda()), slots=listed)) == 0
+    plane, nan = plane.cpu(), torch.isnan(q)
+    got = plane[slots]
+    assert torch.equal(got[~nan], want[~nan]) and bool(((got[nan] & 0x7f) == 0x7f).all())
+    plane[slots] = 0xEE
+    assert bool((plane == 0xEE).all())
+
+
+# Steps of e4m3 rows are 8 a block, of the others 4.  1035 blocks stay for up to eight steps, then there are 4144; listed e4m3 rows have 591 at any
+# of these sizes.
 @pytest.mark.parametrize("kv_format,n", [("fp8", 8 * 8288 - 1), ("fp8", 8 * 8288 + 1), ("mxfp4", 4 * 8288 + 1), ("hybrid", 4 * 8288 + 1), ("fp8", 200001)])
 def test_append_rows_around_the_wave_rule(pkg, kv_format, n):
     from amd_optimization_challenge_b200 import inputs
