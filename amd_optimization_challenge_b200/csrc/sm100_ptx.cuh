@@ -178,8 +178,8 @@ __device__ __forceinline__ void umma_f8_elect(uint32_t d_tmem, uint64_t a_desc, 
 }
 // Four of them behind one election: D, A and B move by D_STEP columns, A_STEP and B_STEP bytes from one to the next; `first` for the first
 // and `rest` for the others: whether D is accumulated into.  The steps are immediates, so that only the first descriptors have to be
-// brought into uniform registers: 16 MMAs of M = 128, K = 32, N = 16 from one idle warp take 918 cycles one by one and 802 so, which is what
-// the tensor core needs for them (977 and 961 with N = 64).
+// brought into uniform registers: 16 MMAs of M = 128, K = 32, N = 16 from one idle warp take 918 cycles one by one and 802 so, 39 each and
+// some 190 from the last one to the commit's arrival (977 and 961 with N = 64, 48 each).
 template <int D_STEP, int A_STEP, int B_STEP>
 __device__ __forceinline__ void umma_f8_x4_elect(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t first, uint32_t rest) {
     static_assert(A_STEP % 16 == 0 && B_STEP % 16 == 0, "descriptors count in 16 bytes");
