@@ -211,18 +211,18 @@ cudaError_t launch_waves(const AppendParams& p, long long steps, int waves, cuda
 }
 // Seven blocks on an SM: up to eight steps per block of a single wave the blocks stay and loop (unlisted e4m3, 16384 rows 5.7 us, 7.2 with
 // a second wave); beyond that four waves even out what the blocks take (131072 rows 40.3 us, 44.5 with one).
-// Listed rows of an e4m3 cache have the slot's load in front of each step: one wave of four blocks that fetch a step ahead takes them.  Up to six
-// blocks on an SM have one step each, nothing to fetch ahead, and more bytes in flight without (us, seven blocks and four ahead, rows in
-// L2 | in HBM: 512 rows 1.47 and 1.56 | 2.04 and 2.09, 4736 2.85 and 3.03 | 3.40 and 3.65, 6000 3.50 and 3.28 | 3.95 and 4.28,
-// 7104 3.95 and 3.52 | 4.44 and 4.49).  Above that it is the faster one, but for two to three steps a block of rows in HBM (7400
-// 4.18 and 3.52 | 4.59 and 4.51, 9000 4.63 and 3.93 | 5.00 and 4.86, 12000 4.86 and 4.55 | 5.61 and 5.82, 16384 6.06 and 5.61 | 6.98 and
-// 6.98, 24000 7.86 and 7.43 | 8.97 and 8.99, 50000 18.0 and 16.4 | 18.3 and 16.5, 131072 41.0 and 40.4 | 40.6 and 40.5, 500000
-// 157 and 150 | 157 and 150).
+// Listed rows of an e4m3 cache have the slot's load in front of each step: one wave of four blocks that fetch a step ahead takes them.  Up to
+// five blocks on an SM have one step each, nothing to fetch ahead, and more bytes in flight without (us, seven blocks and four ahead, rows that
+// a kernel has just written, i.e. in L2 | in HBM: 512 rows 1.47 and 1.56 | 2.04 and 2.09, 4736 2.88 and 3.06 | 3.38 and 3.63, 5500 3.27 and 3.27 |
+// 3.71 and 4.14).  Above that four are faster for rows in L2, and for rows in HBM from 7400 on but for two to three steps a block (6000
+// 3.49 and 3.40 | 3.91 and 4.26, 7104 3.93 and 3.60 | 4.38 and 4.46, 7400 4.28 and 3.71 | 4.59 and 4.51, 9000 4.59 and 4.01 | 5.00 and 4.86, 12000
+// 4.89 and 4.61 | 5.61 and 5.82, 16384 6.14 and 5.86 | 6.98 and 6.98, 24000 8.36 and 8.27 | 8.97 and 8.99, 50000 17.8 and 16.2 |
+// 18.3 and 16.5, 131072 41.0 and 40.3 | 40.6 and 40.5, 500000 157 and 149 | 157 and 150).
 template <int KVFMT>
 cudaError_t launch_format(const AppendParams& p, cudaStream_t stream) {
     const long long steps = (p.n + block_rows(KVFMT) - 1) / block_rows(KVFMT);
     constexpr bool AHEAD = KVFMT == KV_E4M3;
-    if (AHEAD && p.slots && steps > 148 * 6) return launch_waves<KVFMT, true, AHEAD>(p, steps, 1, stream);
+    if (AHEAD && p.slots && steps > 148 * 5) return launch_waves<KVFMT, true, AHEAD>(p, steps, 1, stream);
     const int waves = steps <= 8 * 148 * resident(false) ? 1 : 4;
     return p.slots ? launch_waves<KVFMT, true, false>(p, steps, waves, stream) : launch_waves<KVFMT, false, false>(p, steps, waves, stream);
 }

@@ -666,7 +666,7 @@ def test_append_casts_special_values_as_the_division_does(pkg, scale):
     assert torch.equal(got[~nan], want[~nan]) and bool(((got[nan] & 0x7f) == 0x7f).all())
 
 
-# The same where rows are fetched a step ahead: listed, beyond 7104 of them, 4728 a step of the grid; special rows in each of three
+# The same where rows are fetched a step ahead: listed, beyond 5920 of them, 4728 a step of the grid; special rows in each of three
 # steps, and a slot list that begins on and off a 16-byte boundary.
 @pytest.mark.parametrize("scale,off", [(0.01, 0), (1.0, 3), (2.0 ** -100, 1), (2.0 ** 100, 2)])
 def test_append_of_listed_rows_casts_special_values_in_every_step(pkg, scale, off):

@@ -79,9 +79,9 @@ def test_append_matches_host_quantisers_at_shuffled_slots(pkg):
     assert int(st) == 1
 
 
-@pytest.mark.parametrize("n", [1, 9, 4736, 4737, 7104, 7105, 9456, 9457, 9473, 14185, 16576, 16577, 70001])
+@pytest.mark.parametrize("n", [1, 9, 4736, 4737, 5920, 5921, 9456, 9457, 9473, 14185, 16576, 16577, 70001])
 def test_listed_e4m3_rows_around_the_steps_of_a_wave(pkg, n):
-    """Listed rows (fetched a step ahead beyond 7104 of them, a wave of 4728 at a time) against unlisted ones, bytes of the same rows in
+    """Listed rows (fetched a step ahead beyond 5920 of them, a wave of 4728 at a time) against unlisted ones, bytes of the same rows in
     another order; single slots outside the cache, the first and the last of the list among them, are left out and reported."""
     g = torch.Generator(device="cuda").manual_seed(n)
     rows = torch.randn(n, 576, dtype=torch.bfloat16, generator=g, device="cuda")
@@ -139,14 +139,14 @@ def test_blocks_that_stay_for_several_steps_are_on_the_gpu_together(pkg, kv_form
     assert grid <= -(-n // (8 if kv_format == "fp8" else 4)) + 1
 
 
-@pytest.mark.parametrize("n", [1, 8, 9, 4736, 4737, 7104, 7105])
-def test_up_to_six_blocks_on_an_sm_have_one_step_each(pkg, n):
-    """Listed e4m3 rows: what four blocks on an SM would take in two steps is one where six can have it."""
+@pytest.mark.parametrize("n", [1, 8, 9, 4736, 4737, 5920, 5921])
+def test_up_to_five_blocks_on_an_sm_have_one_step_each(pkg, n):
+    """Listed e4m3 rows: what four blocks on an SM would take in two steps is one where five can have it."""
     planes = torch.empty(n, 576, dtype=torch.uint8, device="cuda"), torch.full((1,), 0.01, device="cuda")
     rows, slots = torch.zeros(n, 576, dtype=torch.bfloat16, device="cuda"), torch.arange(n, dtype=torch.int32, device="cuda")
     grid, held, sms = _captured_launch(lambda: pkg.kv_append(rows, "fp8", planes, slots=slots))
     steps = -(-n // 8)
-    assert sms == 148 and (held, grid) == ((7, steps + 1) if steps <= 6 * sms else (4, 4 * sms))
+    assert sms == 148 and (held, grid) == ((7, steps + 1) if steps <= 5 * sms else (4, 4 * sms))
 
 
 @pytest.mark.parametrize("kv_format,q_format", [("fp8", "fp8"), ("mxfp4", "bf16"), ("hybrid", "fp8")])
